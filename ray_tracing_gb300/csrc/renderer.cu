@@ -1100,7 +1100,6 @@ struct rtgb_renderer {
         for (int b = 0; b < mb; ++b) {
             launch_trace(d_fp, scene, paths, d_counters, b, sh[deep_bvh(scene) ? 14 : 1], stream);
             mark(k);
-            launch_reset_counters(d_counters, b, stream);
             const bool pbr_scene = scene.openpbr_count > 0;
             if (h_fp.sort_from_bounce <= b) launch_shade_sort(d_fp, scene, paths, d_counters, b, sh[1].grid, stream);
             launch_shade(d_fp, scene, paths, d_counters, b, sh[pbr_scene ? 7 : 2], sh[13], stream);
@@ -1267,7 +1266,7 @@ struct rtgb_renderer {
         }
         RTGB_CHECK(cudaGetLastError());
         RTGB_CHECK(cudaEventRecord(ev_stop, stream));
-        RTGB_CHECK(cudaMemcpyAsync(h_counters, d_counters, sizeof(Counters), cudaMemcpyDeviceToHost, stream));
+        RTGB_CHECK(cudaMemcpyAsync(h_counters, d_counters, offsetof(Counters, lengths), cudaMemcpyDeviceToHost, stream));
 
         // capture_launch_history (radiance_launch_setup.cpp:122-136); the
         // frame buffers swap instead of copying into history.

@@ -57,7 +57,7 @@ __global__ void __launch_bounds__(kSortBlock) k_bucket_count(const FrameParams* 
     __syncthreads();
     const int in = bounce & 1;
     int begin, end;
-    chunk_of(counters->active[in], begin, end);
+    chunk_of(counters->lengths[bounce].next, begin, end);
     const int lane = static_cast<int>(threadIdx.x) & 31;
     for (int i = begin + static_cast<int>(threadIdx.x); i < end; i += blockDim.x) {
         const int key = shade_key(s, P.hit[P.queue[in][i]]);
@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(kSortBlock) k_bucket_scatter(const FrameParams
     __syncthreads();
     const int in = bounce & 1;
     int begin, end;
-    chunk_of(counters->active[in], begin, end);
+    chunk_of(counters->lengths[bounce].next, begin, end);
     const int lane = static_cast<int>(threadIdx.x) & 31;
     for (int i = begin + static_cast<int>(threadIdx.x); i < end; i += blockDim.x) {
         const int key = P.sort_key[i];

@@ -45,30 +45,72 @@ RTGB_D void record_decision(const Paths& P, const FrameParams& fp, long long pat
     P.codes[path * fp.max_bounces + bounce] |= bits << kDecisionShift;
 }
 
-// Warp-aggregated queue append: one atomic per warp.
-RTGB_D void queue_push(int* queue, int* count, int value, bool pred) {
+// Queue appends, one atomic per warp for up to two queues whose lengths share
+// eight bytes (`lengths`: the low word counts `qa`, the high word `qb`). The
+// lengths' words are what a frame's largest kernels hammer: same-address
+// atomics retire at about one a clock, and an atomic per queue and warp took
+// as long as shading the terrain's 3.2 M primary hits and misses did. (One
+// atomic per block, behind barriers, measured slower from the second bounce
+// on: the block waits for its slowest warp every iteration.)
+RTGB_D void append_pair(int* qa, int* qb, int* lengths, int value, bool a, bool b) {
+    const unsigned active = __activemask();
+    const unsigned ma = __ballot_sync(active, a), mb = __ballot_sync(active, b);
+    if ((ma | mb) == 0) return;
+    const int lane = threadIdx.x & 31;
+    const int leader = __ffs(active) - 1;
+    unsigned long long base = 0;
+    if (lane == leader) {
+        base = atomicAdd(reinterpret_cast<unsigned long long*>(lengths),
+            static_cast<unsigned long long>(__popc(ma)) | static_cast<unsigned long long>(__popc(mb)) << 32);
+    }
+    base = __shfl_sync(active, base, leader);
+    const unsigned below = (1u << lane) - 1u;
+    if (a) qa[static_cast<unsigned>(base) + __popc(ma & below)] = value;
+    if (b) qb[static_cast<unsigned>(base >> 32) + __popc(mb & below)] = value;
+}
+RTGB_D void append(int* queue, int* length, int value, bool pred) {
     const unsigned active = __activemask();
     const unsigned mask = __ballot_sync(active, pred);
     if (mask == 0) return;
     const int lane = threadIdx.x & 31;
     const int leader = __ffs(mask) - 1;
     int base = 0;
-    if (lane == leader) base = atomicAdd(count, __popc(mask));
+    if (lane == leader) base = atomicAdd(length, __popc(mask));
     base = __shfl_sync(active, base, leader);
     if (pred) queue[base + __popc(mask & ((1u << lane) - 1u))] = value;
 }
+// A run of `n` entries value, value + 1, ... per thread. The lanes that are
+// active together share one atomic.
+RTGB_D void append_run(int* queue, int* length, int value, int n) {
+    const unsigned active = __activemask();
+    const int lane = threadIdx.x & 31;
+    const int total = static_cast<int>(__reduce_add_sync(active, static_cast<unsigned>(n)));
+    if (total == 0) return;
+    const int leader = __ffs(active) - 1;
+    int before = 0;  // entries of the active lanes below this one
+    for (int bit = 0; bit < 4; ++bit) {  // n <= kMaxReuseSources < 16
+        before += __popc(__ballot_sync(active, (n >> bit & 1) != 0) & ((1u << lane) - 1u)) << bit;
+    }
+    int base = 0;
+    if (lane == leader) base = atomicAdd(length, total);
+    base = __shfl_sync(active, base, leader);
+    for (int k = 0; k < n; ++k) queue[base + before + k] = value + k;
+}
 
-RTGB_D void count_add(unsigned long long* counter, unsigned long long v) {
-    // one atomic per thread with work; called once per thread at kernel end
-    if (v) atomicAdd(counter, v);
+// Adds every lane's `v` to a frame counter, one atomic per warp; the whole warp
+// calls it, at kernel end. One per thread made the counter's word the launch's
+// critical path: 60,000 to 120,000 same-address atomics of a persistent grid
+// retire at about one a clock, 30 to 60 us whatever the launch traced.
+RTGB_D void count_add(unsigned long long* counter, unsigned v) {
+    const unsigned sum = __reduce_add_sync(0xffffffffu, v);
+    if ((threadIdx.x & 31) == 0 && sum != 0) atomicAdd(counter, static_cast<unsigned long long>(sum));
 }
 
 struct ShadeCtx {
     const FrameParams& fp;
     const DeviceScene& s;
     int overflow;
-    unsigned long long vis_rays;
-    unsigned long long restir_runs;
+    unsigned vis_rays;
     const float* cdf;    // the ReSTIR candidates' light CDF: shared-memory copy when it fits, else global
     int cdf_count;       // its length: analytic lights, or the emissive list (FrameParams::restir_emissive)
 };
@@ -562,13 +604,20 @@ RTGB_D int subsurface_step(const Paths& P, int path, int sss, const Hit& h, uint
 // path stops there: the ones that scatter are queued for k_scatter, which
 // samples the BSDF from the same RNG state, so each kernel carries only half
 // of the OpenPBR code (evaluation here, sampling there) and fewer registers.
+//
+// Six blocks an SM (80 registers, some spills) for the legacy instance too: it
+// waits on its scattered path-stream loads (DRAM 35 %, issue 35 % at four
+// blocks), and the shading of the Cornell box (64 spp, depth 8) takes 1.47 ms
+// against 1.54 at four or five blocks, the 1280 x 720 final room 2.28 against
+// 2.47 / 2.35 ms.
 template <bool kPbr, bool kSplit = false>
-__global__ void __launch_bounds__(128, kSplit ? 6 : 1) k_shade(const FrameParams* __restrict__ fpp, DeviceScene s, Paths P,
+__global__ void __launch_bounds__(128, 6) k_shade(const FrameParams* __restrict__ fpp, DeviceScene s, Paths P,
     Counters* counters, int bounce) {
     const FrameParams& fp = *fpp;
     const int in = bounce & 1;
     const int out = in ^ 1;
-    const int count = counters->active[in];
+    const int count = counters->lengths[bounce].next;
+    QueueLengths* const filled = &counters->lengths[bounce + 1];
     const bool restir_bounce = fp.restir_enabled != 0 && bounce == 0;
     const int* __restrict__ order = bounce >= fp.sort_from_bounce ? P.sorted : P.queue[in];
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
@@ -698,6 +747,7 @@ __global__ void __launch_bounds__(128, kSplit ? 6 : 1) k_shade(const FrameParams
         P.rad[path] = f4(st.rad, 0.0f);
         P.rng[path] = rng;
         if (keep) store_path(P, path, st);
+        bool any_shadow = false;
         // the random walk scaled the throughput k_scatter starts from
         if (kSplit && to_scatter && thr_changed) P.thr[path] = f4(st.thr, st.prev_pdf);
         if (deferred) {
@@ -711,7 +761,7 @@ __global__ void __launch_bounds__(128, kSplit ? 6 : 1) k_shade(const FrameParams
                 (em ? P.sh_d[1] : P.sh_d[0])[path] = em ? sh_d[1] : sh_d[0];
             }
         } else {
-            const bool any_shadow = sh_c[0].w != 0.0f || sh_c[1].w != 0.0f;
+            any_shadow = sh_c[0].w != 0.0f || sh_c[1].w != 0.0f;
             for (int k = 0; k < 2; ++k) {
                 if (sh_c[k].w != 0.0f) {
                     P.sh_o[k][path] = sh_o[k];
@@ -719,11 +769,14 @@ __global__ void __launch_bounds__(128, kSplit ? 6 : 1) k_shade(const FrameParams
                 }
                 if (any_shadow) P.sh_c[k][path] = sh_c[k];
             }
-            queue_push(P.shadow_queue, &counters->shadow, path, any_shadow);
         }
-        queue_push(P.queue[out], &counters->active[out], path, keep);
-        queue_push(P.restir_queue, &counters->restir, path, deferred);
-        if constexpr (kSplit) queue_push(P.scatter_queue, &counters->scatter, path, to_scatter);
+        if constexpr (kSplit) {
+            append_pair(P.scatter_queue, P.shadow_queue, &filled->scatter, path, to_scatter, any_shadow);
+            append(P.queue[out], &filled->next, path, keep);
+        } else {
+            append_pair(P.queue[out], P.shadow_queue, &filled->next, path, keep, any_shadow);
+        }
+        append(P.restir_queue, &counters->restir, path, deferred);
     }
 }
 
@@ -735,7 +788,8 @@ __global__ void __launch_bounds__(128, 6) k_scatter(const FrameParams* __restric
     Counters* counters, int bounce) {
     const FrameParams& fp = *fpp;
     const int out = (bounce & 1) ^ 1;
-    const int count = counters->scatter;
+    QueueLengths* const filled = &counters->lengths[bounce + 1];
+    const int count = filled->scatter;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
         const int path = P.scatter_queue[i];
         const float4 hr = P.hit[path];
@@ -761,7 +815,7 @@ __global__ void __launch_bounds__(128, 6) k_scatter(const FrameParams* __restric
         }
         P.rng[path] = rng;
         if (keep) store_path(P, path, st);
-        queue_push(P.queue[out], &counters->active[out], path, keep);
+        append(P.queue[out], &filled->next, path, keep);
     }
 }
 
@@ -799,7 +853,7 @@ __global__ void __launch_bounds__(128, 6) k_restir_ris(const FrameParams* __rest
     if (count == 0) return;
     int cdf_count = 0;
     const float* cdf = stage_cdf(fp, s, sh, cdf_count);
-    ShadeCtx ctx{fp, s, 0, 0ull, 0ull, cdf, cdf_count};
+    ShadeCtx ctx{fp, s, 0, 0u, cdf, cdf_count};
     constexpr int bounce = 0;
     const bool bsdf_avail = bounce + 1 < fp.max_bounces;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
@@ -826,10 +880,7 @@ __global__ void __launch_bounds__(128, 6) k_restir_ris(const FrameParams* __rest
         P.rng[path] = rng;
         P.res_meta[path] = pack_meta(nsrc, selected_src, canonical);
         for (int k = 0; k < nsrc; ++k) P.res_src[k * P.src_stride + path] = make_int2(src_index[k], mult[k]);
-        const bool bias = fp.restir_bias == 1 && r.valid != 0;
-        for (int k = 0; k < kMaxSources; ++k) {
-            queue_push(P.vis_queue, &counters->vis, (path << 4) | k, bias && k < nsrc);
-        }
+        append_run(P.vis_queue, &counters->vis, path << 4, fp.restir_bias == 1 && r.valid != 0 ? nsrc : 0);
     }
 }
 
@@ -839,7 +890,7 @@ __global__ void __launch_bounds__(128) k_restir_vis(const FrameParams* __restric
     const FrameParams& fp = *fpp;
     const FrameBufs hist = fp.hist;
     const int count = counters->vis;
-    ShadeCtx ctx{fp, s, 0, 0ull, 0ull, nullptr, 0};
+    ShadeCtx ctx{fp, s, 0, 0u, nullptr, 0};
     constexpr int bounce = 0;
     const bool bsdf_avail = bounce + 1 < fp.max_bounces;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
@@ -863,10 +914,10 @@ __global__ void __launch_bounds__(128) k_restir(const FrameParams* __restrict__ 
     const FrameParams& fp = *fpp;
     FrameBufs cur = fp.cur;
     const int count = counters->restir;
-    ShadeCtx ctx{fp, s, 0, 0ull, 0ull, nullptr, 0};
+    ShadeCtx ctx{fp, s, 0, 0u, nullptr, 0};
     constexpr int bounce = 0;
-    const int out = 1;
-    unsigned long long runs = 0;
+    unsigned runs = 0;
+    QueueLengths* const filled = &counters->lengths[bounce + 1];
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
         const int path = P.restir_queue[i];
         const float4 hr = P.hit[path];
@@ -903,8 +954,12 @@ __global__ void __launch_bounds__(128) k_restir(const FrameParams* __restrict__ 
             P.sh_d[rs][path] = sh_d1;
         }
         if (any_shadow) P.sh_c[rs][path] = sh_c1;
-        queue_push(P.shadow_queue, &counters->shadow, path, any_shadow);
-        queue_push(P.queue[out], &counters->active[out], path, keep);
+        if constexpr (kPbr) {
+            append(P.shadow_queue, &filled->shadow_pbr, path, any_shadow);
+            append(P.queue[1], &filled->next, path, keep);
+        } else {
+            append_pair(P.queue[1], P.shadow_queue, &filled->next, path, keep, any_shadow);
+        }
     }
     count_add(&counters->restir_pixels, runs);
     (void)ctx;

@@ -72,8 +72,15 @@ __global__ void __launch_bounds__(256) k_raygen(const FrameParams* __restrict__ 
             base[i] = z;
         }
     }
+    if (blockIdx.x == 0) {
+        for (int b = threadIdx.x; b <= fp.max_bounces; b += blockDim.x) {
+            counters->lengths[b] = QueueLengths{b == 0 ? static_cast<int>(n) : 0, 0, 0, 0};
+        }
+        for (int b = threadIdx.x; b < 64; b += blockDim.x) counters->shadow_bounce[b] = 0;
+    }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        counters->active[0] = static_cast<int>(n);
+        counters->restir = 0;
+        counters->vis = 0;
         counters->rays[0] = 0;
         counters->rays[1] = 0;
         counters->rays[2] = 0;
@@ -95,18 +102,18 @@ RTGB_D int stage_nodes4(const DeviceScene& s, float4* smem4) {
 constexpr int kStagedBytes = kStagedNodes4 * kNode4 * static_cast<int>(sizeof(float4));
 
 // intersect_scene (programs.cu:1654-1757) + intersect_analytic_lights (:795-813).
-// kDeep: the instance for deep hierarchies (deep_bvh), held to 80 registers so
-// six blocks share an SM.
+// kDeep: the instance for deep hierarchies (deep_bvh), held to 64 registers so
+// eight blocks share an SM.
 template <bool kDeep>
-__global__ void __launch_bounds__(128, kDeep ? 6 : 1) k_trace(const FrameParams* __restrict__ fpp, DeviceScene s, Paths P,
+__global__ void __launch_bounds__(128, kDeep ? 8 : 6) k_trace(const FrameParams* __restrict__ fpp, DeviceScene s, Paths P,
     Counters* counters, int bounce) {
     extern __shared__ float4 smem4[];
     const int staged = stage_nodes4(s, smem4);
     const int in = bounce & 1;
-    const int count = counters->active[in];
+    const int count = counters->lengths[bounce].next;
     if (blockIdx.x == 0 && threadIdx.x == 0 && bounce < 64) counters->bounce_active[bounce] = count;
     int overflow = 0;
-    unsigned long long traced = 0;
+    unsigned traced = 0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
         const int path = P.queue[in][i];
         const float3 o = xyz(P.ray_o[path]);
@@ -147,14 +154,15 @@ __global__ void __launch_bounds__(128, kDeep ? 6 : 1) k_trace(const FrameParams*
 // is_occluded (programs.cu:1759-1762) for the bounce's NEE samples; visible
 // contributions are added in slot order (emissive geometry, then analytic).
 template <bool kDeep>
-__global__ void __launch_bounds__(128, kDeep ? 6 : 1) k_shadow(const FrameParams* __restrict__ fpp, DeviceScene s, Paths P,
+__global__ void __launch_bounds__(128, kDeep ? 8 : 6) k_shadow(const FrameParams* __restrict__ fpp, DeviceScene s, Paths P,
     Counters* counters, int bounce) {
     extern __shared__ float4 smem4[];
     const int staged = stage_nodes4(s, smem4);
     const FrameParams& fp = *fpp;
-    const int count = counters->shadow;
+    const QueueLengths& filled = counters->lengths[bounce + 1];
+    const int count = s.openpbr_count > 0 ? filled.shadow_pbr : filled.shadow;
     int overflow = 0;
-    unsigned long long traced = 0;
+    unsigned traced = 0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
         const int path = P.shadow_queue[i];
         float3 rad = xyz(P.rad[path]);
@@ -285,20 +293,6 @@ __global__ void __launch_bounds__(256) k_resolve(const FrameParams* __restrict__
         cur.normal[pix] = make_float4(hn.x + (cn.x - hn.x) * blend, hn.y + (cn.y - hn.y) * blend,
             hn.z + (cn.z - hn.z) * blend, hn.w + (cn.w - hn.w) * blend);
         cur.depth[pix] = hd + (cd - hd) * blend;
-    }
-}
-
-// Clears the next bounce's queue length and the shadow / ReSTIR queue lengths.
-__global__ void k_reset_counters(Counters* counters, int bounce) {
-    if (threadIdx.x == 0) {
-        counters->active[(bounce & 1) ^ 1] = 0;
-        counters->shadow = 0;
-        counters->restir = 0;
-        counters->vis = 0;
-        counters->scatter = 0;
-        if (bounce == 0) {
-            for (int b = 0; b < 64; ++b) counters->shadow_bounce[b] = 0;
-        }
     }
 }
 
@@ -434,10 +428,6 @@ void query_launch_shapes(int sm_count, LaunchShape* shapes) {
     shapes[7] = query_shade_pbr_shape(sm_count);
     shapes[13] = query_scatter_pbr_shape(sm_count);
     query_restir_pbr_shapes(sm_count, shapes);
-}
-
-void launch_reset_counters(Counters* counters, int bounce, cudaStream_t stream) {
-    k_reset_counters<<<1, 32, 0, stream>>>(counters, bounce);
 }
 
 void launch_direction_debug(const CameraDev& cam, uint8_t* rgba, cudaStream_t stream) {

@@ -57,22 +57,34 @@ struct Paths {
     int* scatter_queue;      // paths whose BSDF sampling runs in k_scatter (split OpenPBR shading)
 };
 
-struct Counters {
-    int active[2];
+// Lengths of the queues one bounce fills, zeroed by k_raygen: `next` the paths
+// that go on, `shadow` its shadow rays, `scatter` the paths k_scatter samples.
+// The two words a kernel mostly appends to together share eight aligned bytes
+// so that one atomic takes places in both queues (append_pair): legacy scenes
+// count shadow rays in `shadow`, beside `next`, OpenPBR ones in `shadow_pbr`,
+// beside `scatter`.
+struct alignas(128) QueueLengths {
+    int next;
     int shadow;
+    int scatter;
+    int shadow_pbr;
+};
+
+struct Counters {
     int error;
-    unsigned long long rays[4];  // primary, extension, shadow, restir visibility
     int overflow;
     int denoise_error;                // a denoiser kernel's bounded wait ran out
     int gave_up;                      // this frame's loops that reached their bound (LoopBounds)
-    int pad;
-    unsigned long long cum_rays[4];  // running totals since the counters were last cleared
-    int bounce_active[64];           // paths entering each bounce of the last frame
+    unsigned long long rays[4];       // primary, extension, shadow, restir visibility
+    unsigned long long cum_rays[4];   // running totals since the counters were last cleared
+    int bounce_active[64];            // paths entering each bounce of the last frame
     unsigned long long restir_pixels; // paths that ran ReSTIR DI in the last frame
-    int restir;                       // ReSTIR queue length
-    int vis;                          // bias-correction ray queue length
     unsigned long long shadow_bounce[64];  // shadow rays traced per bounce
-    int scatter;                      // scatter queue length (split OpenPBR shading)
+    // device only (the host's copy ends here): lengths[b].next paths enter
+    // bounce b, which fills the rest of lengths[b + 1]
+    QueueLengths lengths[65];
+    alignas(128) int restir;          // ReSTIR queue length
+    alignas(128) int vis;             // bias-correction ray queue length
 };
 
 struct FrameParams {
@@ -132,7 +144,6 @@ void launch_restir(const FrameParams* fp, DeviceScene scene, Paths paths, Counte
 void launch_finalize(const FrameParams* fp, Paths paths, Counters* counters, LaunchShape shape, cudaStream_t stream);
 void launch_resolve(const FrameParams* fp, LaunchShape shape, cudaStream_t stream);
 void launch_direction_debug(const CameraDev& cam, uint8_t* rgba, cudaStream_t stream);
-void launch_reset_counters(Counters* counters, int bounce, cudaStream_t stream);
 // Persistent grid sizes: SM count x resident blocks per SM for raygen, trace,
 // shade, shadow, finalize, resolve and restir.
 // shapes[0..6]: raygen, trace, shade, shadow, finalize, resolve, restir;
@@ -144,12 +155,12 @@ void query_launch_shapes(int sm_count, LaunchShape* shapes);
 constexpr int kLaunchShapes = 16;
 
 // Scenes whose wide BVH has at least this many nodes (4 MB) trace with the
-// 80-register instances of k_trace / k_shadow, six blocks per SM: their node
-// fetches miss the L1 and wait on L2 / DRAM, and more warps in flight hide
-// that (the 4 M-triangle room: trace 27.8 against 30.3 ms, shadow 20.7 against
-// 22.5 ms per frame); shallow ones keep the 90-register instances, whose
-// traversal is cache-resident and slower with spills (the benchmark frame:
-// 0.588 against 0.600 ms of trace).
+// 64-register instances of k_trace / k_shadow, eight blocks per SM: their node
+// fetches miss the L1 and wait on L2 / DRAM, and more warps in flight hide that
+// (the 4 M-triangle room: trace 22.1 against 22.9 ms, shadow 17.5 against
+// 18.2 ms per frame at six blocks); shallow ones keep 71 registers, six blocks
+// (at eight, with a few spills, the Cornell box's trace takes 1072 against
+// 1043 us; ten blocks are slower for both: 23.7 ms and 1127 us).
 constexpr int kDeepBvhNodes4 = 1 << 15;
 inline bool deep_bvh(const DeviceScene& s) { return s.node4_count >= kDeepBvhNodes4; }
 
