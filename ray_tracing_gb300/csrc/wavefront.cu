@@ -30,6 +30,27 @@ __global__ void k_camera_dirs(CameraDev cam, float4* out) {
     }
 }
 
+// The pixel of queue slot `k` of a camera in tile order: bands of kTileRows
+// rows, in a band tiles of kTileCols columns, in a tile row by row (the last
+// band and a band's last tile are what is left). A warp of primary rays then
+// covers 8 x 4 pixels instead of a 32-pixel row, its lanes visit more of the
+// same nodes, and later bounces inherit the order (8 pixels of a path stream
+// are still 128 contiguous bytes): primary rays of the 1 M-triangle terrain
+// 972 -> 851 us, of the room's four 1080p cameras 2.24 -> 1.96 ms. 16 x 8 tiles
+// measure the same.
+constexpr int kTileCols = 8;
+constexpr int kTileRows = 4;
+RTGB_D int tile_pixel(int k, int width, int height) {
+    const int band = k / (kTileRows * width);
+    const int rows = min(kTileRows, height - band * kTileRows);
+    int r = k - band * kTileRows * width;
+    const int tile = r / (kTileCols * rows);
+    const int cols = min(kTileCols, width - tile * kTileCols);
+    r -= tile * kTileCols * rows;
+    const int y = r / cols;
+    return (band * kTileRows + y) * width + tile * kTileCols + r - y * cols;
+}
+
 // trace_primary_ray (programs.cu:2086-2099) for every path of every camera.
 __global__ void __launch_bounds__(256) k_raygen(const FrameParams* __restrict__ fpp, Paths P, Counters* counters) {
     const FrameParams& fp = *fpp;
@@ -53,7 +74,7 @@ __global__ void __launch_bounds__(256) k_raygen(const FrameParams* __restrict__ 
         P.rng[path] = rng_for(pixel, sample, fp.stream);
         P.aux_n[path] = make_float4(0.0f, 0.0f, 1.0f, 0.0f);
         P.aux_a[path] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        P.queue[0][path] = static_cast<int>(path);
+        P.queue[0][path] = static_cast<int>(cam.path_offset) + (tile_pixel(pixel, cam.width, cam.height) * fp.spp + sample);
         P.sss_mat[path] = -1;
         if (P.res_written) P.res_written[path] = 0;
         if (fp.record_paths) {
