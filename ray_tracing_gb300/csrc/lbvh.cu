@@ -316,41 +316,140 @@ cudaError_t lbvh_build(LbvhScratch& s, int n, BvhNode* nodes, int** sorted_vals,
     return cudaGetLastError();
 }
 
-int collapse_bvh4(const int* children, int n, std::vector<int>& child4, std::vector<int>& ref4) {
-    child4.clear();
-    ref4.clear();
-    if (n < 2) return 0;
-    std::vector<int> source(1, 0);  // binary node behind each BVH4 node, breadth-first
-    source.reserve(static_cast<size_t>(n));
-    for (size_t i = 0; i < source.size(); ++i) {
-        const int p = source[i];
-        int slot = 0;
-        int c4[4] = {kEmptyChild, kEmptyChild, kEmptyChild, kEmptyChild};
-        int r4[4] = {-1, -1, -1, -1};
-        for (int k = 0; k < 2; ++k) {
-            const int ck = children[2 * p + k];
-            if (ck >= 0) {  // internal: its two children become this node's
-                for (int kk = 0; kk < 2; ++kk) {
-                    const int g = children[2 * ck + kk];
-                    r4[slot] = 2 * ck + kk;
-                    if (g >= 0) {
-                        c4[slot] = static_cast<int>(source.size());
-                        source.push_back(g);
-                    } else {
-                        c4[slot] = g;
-                    }
-                    ++slot;
-                }
-            } else {
-                r4[slot] = 2 * p + k;
-                c4[slot] = ck;
-                ++slot;
-            }
-        }
-        child4.insert(child4.end(), c4, c4 + 4);
-        ref4.insert(ref4.end(), r4, r4 + 4);
+namespace {
+
+// The collapse keeps the binary nodes of even depth (the root is depth 0) in
+// breadth-first order: by depth, and within a depth from left to right, which
+// is the order of their indices (a Karras node's index lies inside the leaf
+// range it covers, and ranges of one depth are disjoint). So the numbering is
+// one stable counting-sort pass over half depths.
+constexpr int kLevels = 64;  // prefix lengths grow by at least one a step: depth <= 64, half depth <= 32
+
+// Half the depth of each internal node, -1 at odd depths.
+__global__ void k_half_depth(const int* __restrict__ parent, int nodes, int* __restrict__ level) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= nodes) return;
+    int d = 0;
+    for (int p = parent[i]; p >= 0 && d < 2 * kLevels - 1; p = parent[p]) ++d;
+    level[i] = (d & 1) != 0 ? -1 : d >> 1;
+}
+
+// Per-tile counts of each level (level-major), the word past them zeroed so
+// that the scan leaves the total there.
+__global__ void __launch_bounds__(kSortThreads) k_level_hist(const int* __restrict__ level, int nodes, uint32_t* hist) {
+    __shared__ uint32_t counts[kLevels];
+    if (threadIdx.x < kLevels) counts[threadIdx.x] = 0;
+    __syncthreads();
+    const int base = blockIdx.x * kSortTile;
+    for (int r = 0; r < kSortItems; ++r) {
+        const int i = base + r * kSortThreads + threadIdx.x;
+        if (i < nodes && level[i] >= 0) atomicAdd(&counts[level[i]], 1u);
     }
-    return static_cast<int>(source.size());
+    __syncthreads();
+    if (threadIdx.x < kLevels) hist[threadIdx.x * gridDim.x + blockIdx.x] = counts[threadIdx.x];
+    if (blockIdx.x == 0 && threadIdx.x == 0) hist[kLevels * gridDim.x] = 0;
+}
+
+// The BVH4 number of every even-depth node (ranked in index order as
+// k_sort_scatter ranks equal digits), -1 for the others.
+__global__ void __launch_bounds__(kSortThreads) k_level_rank(const int* __restrict__ level, int nodes,
+    const uint32_t* __restrict__ hist, int* __restrict__ number) {
+    constexpr int kWarps = kSortThreads / 32;
+    __shared__ uint32_t running[kLevels];
+    __shared__ uint32_t warp_counts[kWarps][kLevels];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x < kLevels) running[threadIdx.x] = hist[threadIdx.x * gridDim.x + blockIdx.x];
+    const int base = blockIdx.x * kSortTile;
+    for (int r = 0; r < kSortItems; ++r) {
+        for (int k = threadIdx.x; k < kWarps * kLevels; k += kSortThreads) (&warp_counts[0][0])[k] = 0;
+        __syncthreads();
+        const int i = base + r * kSortThreads + threadIdx.x;
+        const int l = i < nodes ? level[i] : -1;
+        const unsigned int peers = __match_any_sync(0xffffffffu, l);
+        const int rank = __popc(peers & ((1u << lane) - 1u));
+        if (l >= 0 && rank == 0) warp_counts[warp][l] = __popc(peers);
+        __syncthreads();
+        if (i < nodes) {
+            int id = -1;
+            if (l >= 0) {
+                uint32_t at = running[l];
+                for (int w = 0; w < warp; ++w) at += warp_counts[w][l];
+                id = static_cast<int>(at) + rank;
+            }
+            number[i] = id;
+        }
+        __syncthreads();
+        if (threadIdx.x < kLevels) {
+            uint32_t total = 0;
+            for (int w = 0; w < kWarps; ++w) total += warp_counts[w][threadIdx.x];
+            running[threadIdx.x] += total;
+        }
+        __syncthreads();
+    }
+}
+
+// Children and box references of each BVH4 node: the binary node's children,
+// an internal one replaced by its own two.
+__global__ void k_write_bvh4(const int* __restrict__ children, const int* __restrict__ number, int nodes,
+    int4* __restrict__ child4, int4* __restrict__ ref4) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= nodes || number[i] < 0) return;
+    int c4[4], r4[4];
+    int slot = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        c4[k] = kEmptyChild;
+        r4[k] = -1;
+    }
+    for (int k = 0; k < 2; ++k) {
+        const int c = children[2 * i + k];
+        for (int kk = 0; kk < 2; ++kk) {
+            if (c < 0 && kk == 1) break;
+            const int ref = c < 0 ? 2 * i + k : 2 * c + kk;
+            const int g = c < 0 ? c : children[2 * c + kk];
+            const int id = g < 0 ? g : number[g];
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {  // registers: no dynamic indexing
+                if (t == slot) {
+                    c4[t] = id;
+                    r4[t] = ref;
+                }
+            }
+            ++slot;
+        }
+    }
+    child4[number[i]] = make_int4(c4[0], c4[1], c4[2], c4[3]);
+    ref4[number[i]] = make_int4(r4[0], r4[1], r4[2], r4[3]);
+}
+
+}  // namespace
+
+size_t collapse_scratch_bytes(int n) {
+    const size_t nn = static_cast<size_t>(std::max(n, 2));
+    const size_t blocks = static_cast<size_t>(sort_blocks(static_cast<int>(nn)));
+    return 2 * align256(nn * sizeof(int)) + align256((kLevels * blocks + 1) * sizeof(uint32_t));
+}
+
+cudaError_t number_bvh4(const int* parent, int n, void* scratch, const int** count, cudaStream_t stream) {
+    if (n < 2) return cudaErrorInvalidValue;
+    const int nodes = n - 1, blocks = sort_blocks(nodes), threads = 256;
+    int* level = static_cast<int*>(scratch);
+    int* number = reinterpret_cast<int*>(static_cast<char*>(scratch) + align256(static_cast<size_t>(n) * sizeof(int)));
+    uint32_t* hist = reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(number) + align256(static_cast<size_t>(n) * sizeof(int)));
+    k_half_depth<<<(nodes + threads - 1) / threads, threads, 0, stream>>>(parent, nodes, level);
+    k_level_hist<<<blocks, kSortThreads, 0, stream>>>(level, nodes, hist);
+    k_sort_scan<<<1, 1024, 0, stream>>>(hist, kLevels * blocks + 1);
+    k_level_rank<<<blocks, kSortThreads, 0, stream>>>(level, nodes, hist, number);
+    *count = reinterpret_cast<const int*>(hist + static_cast<size_t>(kLevels) * blocks);
+    return cudaGetLastError();
+}
+
+cudaError_t write_bvh4(const int* children, int n, const void* scratch, int* child4, int* ref4, cudaStream_t stream) {
+    const int nodes = n - 1, threads = 256;
+    const int* number = reinterpret_cast<const int*>(static_cast<const char*>(scratch) + align256(static_cast<size_t>(n) * sizeof(int)));
+    k_write_bvh4<<<(nodes + threads - 1) / threads, threads, 0, stream>>>(children, number, nodes,
+        reinterpret_cast<int4*>(child4), reinterpret_cast<int4*>(ref4));
+    return cudaGetLastError();
 }
 
 namespace {

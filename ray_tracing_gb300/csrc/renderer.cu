@@ -139,15 +139,6 @@ struct DevBuf {
     }
 };
 
-// A build-time scratch buffer freed when it leaves scope (cudaFree waits for
-// the work that uses it), also when the build throws.
-struct ScopedBuf : DevBuf {
-    ScopedBuf() = default;
-    ScopedBuf(const ScopedBuf&) = delete;
-    ScopedBuf& operator=(const ScopedBuf&) = delete;
-    ~ScopedBuf() { release(); }
-};
-
 // Timing events destroyed on every exit path.
 struct EventPair {
     cudaEvent_t a = nullptr, b = nullptr;
@@ -233,6 +224,10 @@ struct rtgb_renderer {
     // references into the binary nodes) kept for refits
     DevBuf nodes4, child4, ref4;
     int node4_count = 0;
+    // scene preparation's workspaces, kept between prepares (allocating and
+    // freeing them, with the synchronisation a free implies, was 0.5 ms of a
+    // refit of 200,000 triangles); the light BVH reuses the scene's
+    DevBuf lbvh_mem, collapse_mem, unsorted, light_mem;
     bool accel_valid = false;
     int accel_counts[3] = {-1, -1, -1};
     uint64_t geometry_sig = 0, scene_sig = 0;
@@ -293,6 +288,9 @@ struct rtgb_renderer {
     // graph
     cudaGraphExec_t graph_exec = nullptr;
     long long graph_key[5] = {-1, -1, -1, -1, -1};
+    // the scene the captured launches carry by value: a refit or an update that
+    // leaves every address and count in place keeps the graph
+    DeviceScene graph_scene{};
     long long unet_generation = 0;
 
     void fail_cuda(const CudaFailure& f) {
@@ -342,7 +340,7 @@ struct rtgb_renderer {
             &infinite_analytic, &prims, &nodes, &sorted_keys, &sorted_vals, &frame_mem[0], &frame_mem[1], &path_mem,
             &counters_mem, &fp_mem, &debug_rgba, &openpbr, &analytic_hot, &bvh_children, &bvh_parent, &nodes4, &child4, &ref4,
             &light_guide, &analytic_guide, &material_lum, &light_counts, &mesh_points, &mesh_corners, &mesh_normals,
-            &mesh_texcoords, &mesh_materials, &mesh_protos, &mesh_insts};
+            &mesh_texcoords, &mesh_materials, &mesh_protos, &mesh_insts, &lbvh_mem, &collapse_mem, &unsorted, &light_mem};
         for (DevBuf* b : bufs) b->release();
         for (auto& slot : cam_res) {
             for (auto& r : slot) {
@@ -608,7 +606,6 @@ struct rtgb_renderer {
         else if (geo != geometry_sig) kind = 2;
         else if (sig != scene_sig) kind = 1;
         if (kind != 0) {
-            drop_graph();
             prepared = false;
             accel_valid = false;
             upload_scene(s, kind, meshes);
@@ -708,9 +705,7 @@ struct rtgb_renderer {
                 static_cast<float*>(light_cdf.ensure((prims + 1) * sizeof(float))), ints(light_guide, kGuide + 1),
                 ints(sphere_light, static_cast<size_t>(d.sphere_count)), ints(quad_light, static_cast<size_t>(d.quad_count)),
                 ints(triangle_light, static_cast<size_t>(d.triangle_count)), ints(light_counts, 4)};
-            ScopedBuf scratch;
-            scratch.ensure(light_table_scratch_bytes(static_cast<long long>(prims)));
-            RTGB_CHECK(launch_light_table(src, lt, scratch.p, stream));
+            RTGB_CHECK(launch_light_table(src, lt, light_mem.ensure(light_table_scratch_bytes(static_cast<long long>(prims))), stream));
             int counts[2] = {0, -1};
             RTGB_CHECK(cudaMemcpyAsync(counts, lt.counts, sizeof counts, cudaMemcpyDeviceToHost, stream));
             RTGB_CHECK(cudaStreamSynchronize(stream));
@@ -774,10 +769,8 @@ struct rtgb_renderer {
         const float pad = 1e-5f + 1e-5f * scale;
         d.prim_count = n;
         prim_count = n;
-        ScopedBuf scratch, unsorted;
         unsorted.ensure(static_cast<size_t>(n) * sizeof(PrimRecord));
-        scratch.ensure(lbvh_scratch_bytes(n));
-        LbvhScratch ls = lbvh_carve(scratch.p, n);
+        LbvhScratch ls = lbvh_carve(lbvh_mem.ensure(lbvh_scratch_bytes(n)), n);
         PrimRecord* recs = static_cast<PrimRecord*>(prims.ensure(static_cast<size_t>(n) * sizeof(PrimRecord)));
         launch_prim_records(d, unsorted.as<PrimRecord>(), ls.aabb_lo, ls.aabb_hi, pad, stream);
         RTGB_CHECK(cudaGetLastError());
@@ -807,19 +800,17 @@ struct rtgb_renderer {
                 cudaMemcpyDeviceToDevice, stream));
             RTGB_CHECK(cudaMemcpyAsync(bvh_parent.p, ls.parent, (2 * static_cast<size_t>(n) - 1) * sizeof(int),
                 cudaMemcpyDeviceToDevice, stream));
-            // the wide BVH: collapse the binary hierarchy on the host, boxes filled on the device
-            std::vector<int> children2(2 * static_cast<size_t>(n - 1)), c4, r4;
-            RTGB_CHECK(cudaMemcpyAsync(children2.data(), ls.children, children2.size() * sizeof(int), cudaMemcpyDeviceToHost,
-                stream));
+            // the wide BVH: the binary hierarchy collapsed, then its boxes filled in
+            void* work = collapse_mem.ensure(collapse_scratch_bytes(n));
+            const int* count4 = nullptr;
+            RTGB_CHECK(number_bvh4(ls.parent, n, work, &count4, stream));
+            RTGB_CHECK(cudaMemcpyAsync(&node4_count, count4, sizeof node4_count, cudaMemcpyDeviceToHost, stream));
             RTGB_CHECK(cudaStreamSynchronize(stream));
-            node4_count = collapse_bvh4(children2.data(), n, c4, r4);
-            RTGB_CHECK(cudaMemcpyAsync(child4.ensure(c4.size() * sizeof(int)), c4.data(), c4.size() * sizeof(int),
-                cudaMemcpyHostToDevice, stream));
-            RTGB_CHECK(cudaMemcpyAsync(ref4.ensure(r4.size() * sizeof(int)), r4.data(), r4.size() * sizeof(int),
-                cudaMemcpyHostToDevice, stream));
+            child4.ensure(4 * static_cast<size_t>(node4_count) * sizeof(int));
+            ref4.ensure(4 * static_cast<size_t>(node4_count) * sizeof(int));
+            RTGB_CHECK(write_bvh4(ls.children, n, work, child4.as<int>(), ref4.as<int>(), stream));
             nodes4.ensure(static_cast<size_t>(node4_count) * kNode4 * sizeof(float4));
             RTGB_CHECK(fill_bvh4(nd, child4.as<int>(), ref4.as<int>(), node4_count, nodes4.as<float4>(), stream));
-            RTGB_CHECK(cudaStreamSynchronize(stream));  // the host vectors leave scope
             d.nodes = nd;
             d.node_count = n - 1;
         } else {
@@ -866,9 +857,7 @@ struct rtgb_renderer {
             }
             std::vector<int> leaf(static_cast<size_t>(nf));
             if (nf >= 2) {
-                ScopedBuf ascratch;
-                ascratch.ensure(lbvh_scratch_bytes(nf));
-                LbvhScratch as = lbvh_carve(ascratch.p, nf);
+                LbvhScratch as = lbvh_carve(lbvh_mem.ensure(lbvh_scratch_bytes(nf)), nf);
                 RTGB_CHECK(cudaMemcpyAsync(as.aabb_lo, lo.data(), lo.size() * sizeof(float4), cudaMemcpyHostToDevice, stream));
                 RTGB_CHECK(cudaMemcpyAsync(as.aabb_hi, hi.data(), hi.size() * sizeof(float4), cudaMemcpyHostToDevice, stream));
                 BvhNode* an = static_cast<BvhNode*>(analytic_nodes.ensure(static_cast<size_t>(nf - 1) * sizeof(BvhNode)));
@@ -1249,7 +1238,8 @@ struct rtgb_renderer {
             static_cast<long long>(paths.ray_o != nullptr) | (fp.sort_from_bounce != INT_MAX ? 2ll : 0ll),
             reinterpret_cast<long long>(scene.prims), (denoise_this_frame ? 1ll : 0ll) | (static_cast<long long>(unet_generation) << 1)};
         if (use_graph) {
-            if (!graph_exec || std::memcmp(key, graph_key, sizeof key) != 0) {
+            if (!graph_exec || std::memcmp(key, graph_key, sizeof key) != 0 ||
+                std::memcmp(&scene, &graph_scene, sizeof scene) != 0) {
                 drop_graph();
                 cudaGraph_t graph;
                 RTGB_CHECK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
@@ -1259,6 +1249,7 @@ struct rtgb_renderer {
                 cudaGraphDestroy(graph);
                 RTGB_CHECK(inst);
                 std::memcpy(graph_key, key, sizeof key);
+                std::memcpy(&graph_scene, &scene, sizeof scene);
             }
             RTGB_CHECK(cudaGraphLaunch(graph_exec, stream));
         } else {
