@@ -53,11 +53,13 @@ cudaError_t conv_init();
 cudaError_t launch_conv3x3(const CUtensorMap& map, int n, int h, int w, int cin, const void* weight, const float* bias,
     int cout, int relu, void* y, int y_channels, int y_offset, int* err, int grid_limit, cudaStream_t stream,
     void* pool = nullptr, int up = 0, int stages = 0);
-// Weight (cout x cin x 3 x 3, FP32) and bias gradients of a k_conv3x3 layer
-// (denoiser_train.cu); `partial` holds wgrad_partial_bytes(sms, cout).
-cudaError_t launch_conv3x3_wgrad(const void* x, int n, int h, int w, int cin, const void* dy, int cout, float* dweight,
-    float* dbias, int* err, int sms, cudaStream_t stream, float* partial, size_t partial_bytes);
-size_t wgrad_partial_bytes(int sms, int cout);
+// Weight (cout_used x cin_used x 3 x 3, FP32) and bias gradients of a k_conv3x3
+// layer (denoiser_train.cu); `partial` holds wgrad_partial_bytes of at least
+// min(sms, tiles) CTAs.
+cudaError_t launch_conv3x3_wgrad(const void* x, int n, int h, int w, int cin, const void* dy, int cout, int cin_used,
+    int cout_used, float* dweight, float* dbias, int* err, int sms, cudaStream_t stream, float* partial,
+    size_t partial_bytes);
+size_t wgrad_partial_bytes(int ctas, int cin, int cout);
 
 struct UNet;
 

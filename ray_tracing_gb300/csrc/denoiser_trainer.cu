@@ -16,6 +16,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <string>
@@ -203,21 +204,6 @@ __global__ void k_pack_weights(const float* __restrict__ wsrc, int cout_used, in
     }
 }
 
-// The used block of a layer's padded weight gradient (cout x cin x 9) and its
-// bias gradient into the flat parameter-gradient vector.
-__global__ void k_gather_grad(const float* __restrict__ dw, const float* __restrict__ db, int cout_used, int cin_used,
-    int cin, float* __restrict__ flat) {
-    const int nw = cout_used * cin_used * 9;
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < nw + cout_used; e += gridDim.x * blockDim.x) {
-        if (e < nw) {
-            const int tap = e % 9, i = (e / 9) % cin_used, o = e / (9 * cin_used);
-            flat[e] = dw[(static_cast<long long>(o) * cin + i) * 9 + tap];
-        } else {
-            flat[e] = db[e - nw];
-        }
-    }
-}
-
 // Adam (Kingma & Ba 2015) on the FP32 master parameters, bias-corrected.
 __global__ void k_adam(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
     long long count, float lr, float b1, float b2, float eps, float c1, float c2) {
@@ -252,7 +238,7 @@ struct Trainer {
     __nv_bfloat16* wb[kLayerCount][2] = {};
     float* bias[kLayerCount] = {};       // FP32 bias (forward), padded to cout
     float* zero_bias = nullptr;          // 128 zeros for the input-gradient convolutions
-    float *dw = nullptr, *db = nullptr, *partial = nullptr;
+    float* partial = nullptr;
     size_t partial_bytes = 0;
     // activations (channel-blocked BF16)
     __nv_bfloat16 *t1, *cat1, *p1, *t2, *cat2, *p2, *t3, *t4, *t5, *t6, *out16;
@@ -306,9 +292,9 @@ struct Trainer {
             bias[l] = alloc<float>(L.cout);
         }
         zero_bias = alloc<float>(128);
-        dw = alloc<float>(64 * 128 * 9);
-        db = alloc<float>(64);
-        partial_bytes = wgrad_partial_bytes(sms, 64);
+        for (const LayerSpec& L : kLayers) {
+            partial_bytes = std::max(partial_bytes, wgrad_partial_bytes(sms, L.cin, L.cout));
+        }
         partial = alloc<float>(partial_bytes / sizeof(float));
         const size_t full = static_cast<size_t>(n) * h * w, half = full / 4, quarter = full / 16;
         t1 = alloc<__nv_bfloat16>(full * 32);
@@ -393,11 +379,10 @@ struct Trainer {
     // weight/bias gradients of layer l (x: its input, dz: its masked output gradient) into the flat vector
     void wgrad(int l, const void* x, int hh, int ww, const void* dz) {
         const LayerSpec& L = kLayers[l];
-        check(launch_conv3x3_wgrad(x, n, hh, ww, L.cin, dz, L.cout, dw, db, err, sms, stream, partial, partial_bytes),
+        float* dw = grads + offset[l];
+        check(launch_conv3x3_wgrad(x, n, hh, ww, L.cin, dz, L.cout, L.cin_used, L.cout_used, dw,
+                  dw + static_cast<long long>(L.cout_used) * L.cin_used * 9, err, sms, stream, partial, partial_bytes),
             "wgrad");
-        k_gather_grad<<<grid_of(static_cast<long long>(L.cout_used) * L.cin_used * 9 + L.cout_used), 256, 0, stream>>>(
-            dw, db, L.cout_used, L.cin_used, L.cin, grads + offset[l]);
-        check(cudaGetLastError(), "gather");
     }
 
     // input gradient of layer l: dX (cin channels, written at channel xoff of an xcs tensor) from dz (cout channels)
