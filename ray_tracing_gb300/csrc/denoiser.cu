@@ -105,6 +105,7 @@ struct ConvArgs {
     int* err;
     // fused epilogue variants (k_conv3x3's comment)
     __nv_bfloat16* pool;   // non-null: also write the 2x2 average of the output (dense cout channels)
+    const __nv_bfloat16* mask;  // non-null: keep an output only where this tensor (y_channels, y_offset, as y) is > 0
     int up;                // non-zero: y is twice the input size, each output pixel written 2 x 2
     int stages;            // halo stages in shared memory (conv_stages)
     uint32_t tmem_cols;    // conv_tmem_cols(cout)
@@ -158,6 +159,16 @@ __device__ __forceinline__ void conv_epilogue(const ConvArgs& a, uint32_t acc, i
                 hi = fmaxf(hi, 0.0f);
             }
             packed[k] = pack_bf16x2(lo, hi);
+        }
+        if (a.mask != nullptr && inside) {
+            // the ReLU's backward pass of the layer this gradient belongs to
+            const __nv_bfloat16* mb = a.mask + (out - a.y) + 2 * g * oplane;
+            const uint4 m0 = __ldg(reinterpret_cast<const uint4*>(mb));
+            const uint4 m1 = __ldg(reinterpret_cast<const uint4*>(mb + oplane));
+            const uint32_t m[8] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w};
+            const __nv_bfloat162 zero = __floats2bfloat162_rn(0.0f, 0.0f);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) packed[k] &= __hgt2_mask(*reinterpret_cast<const __nv_bfloat162*>(&m[k]), zero);
         }
         const uint4 q0 = make_uint4(packed[0], packed[1], packed[2], packed[3]);
         const uint4 q1 = make_uint4(packed[4], packed[5], packed[6], packed[7]);
@@ -451,12 +462,13 @@ cudaError_t conv_init() {
 // Launches k_conv3x3; `map` must describe x (conv_input_map).
 cudaError_t launch_conv3x3(const CUtensorMap& map, int n, int h, int w, int cin, const void* weight, const float* bias,
     int cout, int relu, void* y, int y_channels, int y_offset, int* err, int grid_limit, cudaStream_t stream,
-    void* pool, int up, int stages) {
+    void* pool, int up, int stages, const void* mask) {
     const cudaError_t attr = conv_init();
     if (attr != cudaSuccess) return attr;
     if (stages <= 0 || stages > kMaxStages || conv_smem_bytes(cin, cout, stages) > kConvSmem) stages = conv_stages(cin, cout);
     ConvArgs a{n, h, w, cin, cout, y_channels, y_offset, relu, static_cast<const uint4*>(weight), bias,
-        static_cast<__nv_bfloat16*>(y), err, static_cast<__nv_bfloat16*>(pool), up, stages, conv_tmem_cols(cout)};
+        static_cast<__nv_bfloat16*>(y), err, static_cast<__nv_bfloat16*>(pool), static_cast<const __nv_bfloat16*>(mask), up,
+        stages, conv_tmem_cols(cout)};
     const int smem = conv_smem_bytes(cin, cout, stages);
     // resident CTAs per SM: 228 KB of shared memory (1 KB reserved per CTA),
     // 512 TMEM columns (conv_tmem_cols each, so no allocation ever waits),

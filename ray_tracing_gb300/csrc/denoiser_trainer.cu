@@ -6,9 +6,10 @@
 //     (dX = conv(dZ, W^T flipped)), split into launches of <= 64 output
 //     channels;
 //   * weight and bias gradients: k_conv3x3_wgrad (denoiser_train.cu);
-//   * ReLU masks, the backward of 2 x 2 average pooling and of nearest
-//     upsampling, the loss gradient, weight packing and Adam: elementwise
-//     kernels below.
+//   * ReLU masks: in the input-gradient convolutions' epilogue;
+//   * the backward of 2 x 2 average pooling and of nearest upsampling (with
+//     their ReLU masks), the loss gradient, weight packing and Adam:
+//     elementwise kernels below.
 // Gradients flow in BF16 between layers and accumulate in FP32 inside each
 // GEMM; the master parameters and Adam moments are FP32. Batches are n crops
 // of h x w with h and w multiples of 4 (the pooled sizes then halve exactly).
@@ -32,61 +33,50 @@ namespace {
 
 __device__ __forceinline__ float bf2f(__nv_bfloat16 v) { return __bfloat162float(v); }
 
-// Offset of channel c of pixel (img, y, x) in a blocked tensor of `cs` channels.
-__device__ __forceinline__ long long blk(int img, int c, int cs, int h, int w, int y, int x) {
-    return ((((static_cast<long long>(img) * (cs >> 3) + (c >> 3)) * h + y) * w + x) << 3) + (c & 7);
-}
-
 // Loss gradient of mean |out - target| over n x h x w x 3 (log1p radiance):
 // sign / count into channels 0..2 of a 16-channel gradient, 0 elsewhere; the
-// loss sum goes to *loss.
-__global__ void k_loss_grad(const __nv_bfloat16* __restrict__ out16, const float* __restrict__ target, int n, int h,
-    int w, __nv_bfloat16* __restrict__ g16, double* loss) {
-    const long long px = static_cast<long long>(n) * h * w;
+// loss sum goes to *loss. A thread moves a pixel's 16 channels as two 16-byte
+// stores (`hw` pixels per image), a block adds one value to the sum (2-byte
+// stores and an atomic per warp took 58 us for 16 x 256 x 256 pixels).
+__global__ void __launch_bounds__(256) k_loss_grad(const __nv_bfloat16* __restrict__ out16, const float* __restrict__ target,
+    long long px, int hw, __nv_bfloat16* __restrict__ g16, double* loss) {
+    __shared__ double part[8];
     const float inv = 1.0f / static_cast<float>(px * 3);
     double local = 0.0;
     for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < px;
          i += static_cast<long long>(gridDim.x) * blockDim.x) {
-        const int x = static_cast<int>(i % w);
-        const int y = static_cast<int>((i / w) % h);
-        const int img = static_cast<int>(i / (static_cast<long long>(w) * h));
-        for (int c = 0; c < 16; ++c) {
-            float g = 0.0f;
+        const long long img = i / hw, p = i - img * hw;
+        const long long at = (img * 2 * hw + p) * 8;  // the pixel in channel block 0; block 1 is hw pixels on
+        const uint2 q = *reinterpret_cast<const uint2*>(out16 + at);
+        const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&q);
+        __align__(16) __nv_bfloat16 g[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+            float v = 0.0f;
             if (c < 3) {
-                const float d = bf2f(out16[blk(img, c, 16, h, w, y, x)]) - target[i * 3 + c];
+                const float d = bf2f(e[c]) - target[i * 3 + c];
                 local += fabsf(d);
-                g = d > 0.0f ? inv : (d < 0.0f ? -inv : 0.0f);
+                v = d > 0.0f ? inv : (d < 0.0f ? -inv : 0.0f);
             }
-            g16[blk(img, c, 16, h, w, y, x)] = __float2bfloat16_rn(g);
+            g[c] = __float2bfloat16_rn(v);
         }
+        *reinterpret_cast<uint4*>(g16 + at) = *reinterpret_cast<const uint4*>(g);
+        *reinterpret_cast<uint4*>(g16 + at + 8ll * hw) = make_uint4(0, 0, 0, 0);
     }
     for (int off = 16; off > 0; off >>= 1) local += __shfl_down_sync(0xffffffffu, local, off);
-    if ((threadIdx.x & 31) == 0) atomicAdd(loss, local);
-}
-
-// out[c] = g[c] * (y[c] > 0) for c < channels; g, y and out are channel ranges
-// (offset, channel count of the whole tensor) of blocked tensors of n x h x w.
-__global__ void k_relu_mask(const __nv_bfloat16* __restrict__ g, int g_cs, int g_off, const __nv_bfloat16* __restrict__ y,
-    int y_cs, int y_off, __nv_bfloat16* __restrict__ out, int o_cs, int o_off, int channels, int n, int h, int w) {
-    const long long total = static_cast<long long>(n) * h * w * channels;
-    for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total;
-         i += static_cast<long long>(gridDim.x) * blockDim.x) {
-        const int c = static_cast<int>(i % channels);
-        long long r = i / channels;
-        const int x = static_cast<int>(r % w);
-        r /= w;
-        const int yy = static_cast<int>(r % h);
-        const int img = static_cast<int>(r / h);
-        const float gv = bf2f(g[blk(img, g_off + c, g_cs, h, w, yy, x)]);
-        const float yv = bf2f(y[blk(img, y_off + c, y_cs, h, w, yy, x)]);
-        out[blk(img, o_off + c, o_cs, h, w, yy, x)] = __float2bfloat16_rn(yv > 0.0f ? gv : 0.0f);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = local;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w) local += part[w];
+        atomicAdd(loss, local);
     }
 }
 
 // Backward passes on whole 8-channel blocks (every channel count and offset of
 // the U-Net is a multiple of 8): a thread moves one pixel's 8 channels as one
 // 16-byte load per operand, and the index arithmetic is 32-bit on (image,
-// channel block, pixel). k_relu_mask8 computes each element as k_relu_mask.
+// channel block, pixel). (A ReLU alone needs no pass: the input-gradient
+// convolution stores its output masked.)
 __device__ __forceinline__ void unpack8(const uint4& q, float f[8]) {
     const __nv_bfloat16* v = reinterpret_cast<const __nv_bfloat16*>(&q);
 #pragma unroll
@@ -102,23 +92,6 @@ __device__ __forceinline__ uint4 pack8(const float f[8]) {
 // 16-byte unit of channel block `cb` (of `cbs`) at pixel p of image img, hw pixels
 __device__ __forceinline__ long long unit(int img, int cbs, int cb, int hw, int p) {
     return (static_cast<long long>(img) * cbs + cb) * hw + p;
-}
-
-__global__ void k_relu_mask8(const uint4* __restrict__ g, int g_cbs, int g_cb0, const uint4* __restrict__ y, int y_cbs,
-    int y_cb0, uint4* __restrict__ out, int o_cbs, int o_cb0, int blocks, int n, int hw) {
-    const long long total = static_cast<long long>(n) * blocks * hw;
-    for (long long j = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; j < total;
-         j += static_cast<long long>(gridDim.x) * blockDim.x) {
-        const int p = static_cast<int>(j % hw);
-        const int t = static_cast<int>(j / hw);
-        const int cb = t % blocks, img = t / blocks;
-        float gv[8], yv[8], o[8];
-        unpack8(g[unit(img, g_cbs, g_cb0 + cb, hw, p)], gv);
-        unpack8(y[unit(img, y_cbs, y_cb0 + cb, hw, p)], yv);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) o[k] = yv[k] > 0.0f ? gv[k] : 0.0f;
-        out[unit(img, o_cbs, o_cb0 + cb, hw, p)] = pack8(o);
-    }
 }
 
 // Backward of nearest 2x upsampling followed by the ReLU of the layer that
@@ -178,29 +151,45 @@ __global__ void k_pool_backward_mask8(const uint4* __restrict__ g, int g_cbs, in
     }
 }
 
-// Packs FP32 weights (cout_used x cin_used x 3 x 3 at `wsrc`) as
-// rtgb_conv3x3_pack_weights does, [tap][cin/8][cout][8] BF16 with zero
-// padding; with `transposed` the packed kernel is the input-gradient one,
-// W'[i][o][2 - dy][2 - dx], for output channels [o0, o0 + cout) of it
-// (i.e. layer input channels) and input channels = the layer's cout.
-__global__ void k_pack_weights(const float* __restrict__ wsrc, int cout_used, int cin_used, int transposed, int o0,
-    int cout, int cin, __nv_bfloat16* __restrict__ packed) {
-    const int total = 9 * cin * cout;
+// One tensor of a step's weight packing: FP32 weights (cout_used x cin_used x
+// 3 x 3, then the bias, at params + src) as rtgb_conv3x3_pack_weights packs
+// them, [tap][cin/8][cout][8] BF16 with zero padding; with `transposed` the
+// packed kernel is the input-gradient one, W'[i][o][2 - dy][2 - dx], for output
+// channels [o0, o0 + cout) of it (i.e. layer input channels) and input channels
+// = the layer's cout. With `bias` set instead of `packed`, the bias padded to cout.
+struct PackTask {
+    long long src;
+    int cout_used, cin_used, transposed, o0, cout, cin;
+    __nv_bfloat16* packed;
+    float* bias;
+};
+
+// Every layer's packed tensors in one launch, blockIdx.y the task (24 launches
+// and 22 copies of a few KB each were 70 us of device time and most of a small
+// step's launches).
+__global__ void k_pack_weights(const float* __restrict__ params, const PackTask* __restrict__ tasks) {
+    const PackTask t = tasks[blockIdx.y];
+    const float* __restrict__ wsrc = params + t.src;
+    const int total = t.packed != nullptr ? 9 * t.cin * t.cout : t.cout;
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < total; e += gridDim.x * blockDim.x) {
+        if (t.packed == nullptr) {
+            t.bias[e] = e < t.cout_used ? wsrc[static_cast<long long>(t.cout_used) * t.cin_used * 9 + e] : 0.0f;
+            continue;
+        }
         const int j = e & 7;
-        const int o = (e >> 3) % cout;
-        const int b = (e >> 3) / cout % (cin >> 3);
-        const int tap = (e >> 3) / cout / (cin >> 3);
+        const int o = (e >> 3) % t.cout;
+        const int b = (e >> 3) / t.cout % (t.cin >> 3);
+        const int tap = (e >> 3) / t.cout / (t.cin >> 3);
         const int i = b * 8 + j;
         float v = 0.0f;
-        if (!transposed) {
-            if (o < cout_used && i < cin_used) v = wsrc[(static_cast<long long>(o) * cin_used + i) * 9 + tap];
+        if (!t.transposed) {
+            if (o < t.cout_used && i < t.cin_used) v = wsrc[(static_cast<long long>(o) * t.cin_used + i) * 9 + tap];
         } else {
             // packed output channel o = layer input channel o0 + o, packed input i = layer output channel
-            const int li = o0 + o, lo = i;
-            if (li < cin_used && lo < cout_used) v = wsrc[(static_cast<long long>(lo) * cin_used + li) * 9 + (8 - tap)];
+            const int li = t.o0 + o, lo = i;
+            if (li < t.cin_used && lo < t.cout_used) v = wsrc[(static_cast<long long>(lo) * t.cin_used + li) * 9 + (8 - tap)];
         }
-        packed[e] = __float2bfloat16_rn(v);
+        t.packed[e] = __float2bfloat16_rn(v);
     }
 }
 
@@ -237,6 +226,8 @@ struct Trainer {
     __nv_bfloat16* wf[kLayerCount] = {};
     __nv_bfloat16* wb[kLayerCount][2] = {};
     float* bias[kLayerCount] = {};       // FP32 bias (forward), padded to cout
+    PackTask* pack_tasks = nullptr;      // device: what k_pack_weights writes
+    int pack_count = 0;
     float* zero_bias = nullptr;          // 128 zeros for the input-gradient convolutions
     float* partial = nullptr;
     size_t partial_bytes = 0;
@@ -292,6 +283,7 @@ struct Trainer {
             bias[l] = alloc<float>(L.cout);
         }
         zero_bias = alloc<float>(128);
+        list_pack_tasks();
         for (const LayerSpec& L : kLayers) {
             partial_bytes = std::max(partial_bytes, wgrad_partial_bytes(sms, L.cin, L.cout));
         }
@@ -323,8 +315,8 @@ struct Trainer {
         g_p1 = alloc<__nv_bfloat16>(half * 32);
         g1 = alloc<__nv_bfloat16>(full * 32);
         g_t1 = alloc<__nv_bfloat16>(full * 32);
-        loss = alloc<double>(1);
-        err = alloc<int>(1);
+        loss = alloc<double>(2);  // the sum, then the error word: cleared and read as one
+        err = reinterpret_cast<int*>(loss + 1);
         if (conv_init() != cudaSuccess) throw std::string("conv_init");
         cudaDeviceSynchronize();
     }
@@ -335,29 +327,33 @@ struct Trainer {
 
     // packs every layer's forward and input-gradient weights and copies the biases
     void pack() {
+        k_pack_weights<<<dim3(16, static_cast<unsigned>(pack_count)), 256, 0, stream>>>(params, pack_tasks);
+        check(cudaGetLastError(), "pack");
+    }
+
+    void list_pack_tasks() {
+        std::vector<PackTask> tasks;
         for (int l = 0; l < kLayerCount; ++l) {
             const LayerSpec& L = kLayers[l];
-            const float* W = params + offset[l];
-            k_pack_weights<<<grid_of(9LL * L.cin * L.cout), 256, 0, stream>>>(W, L.cout_used, L.cin_used, 0, 0, L.cout,
-                L.cin, wf[l]);
+            tasks.push_back({offset[l], L.cout_used, L.cin_used, 0, 0, L.cout, L.cin, wf[l], nullptr});
             for (int k = 0; k * 64 < L.cin; ++k) {
                 const int oc = L.cin - 64 * k < 64 ? L.cin - 64 * k : 64;
-                k_pack_weights<<<grid_of(9LL * L.cout * oc), 256, 0, stream>>>(W, L.cout_used, L.cin_used, 1, 64 * k, oc,
-                    L.cout, wb[l][k]);
+                tasks.push_back({offset[l], L.cout_used, L.cin_used, 1, 64 * k, oc, L.cout, wb[l][k], nullptr});
             }
-            check(cudaMemsetAsync(bias[l], 0, L.cout * sizeof(float), stream), "bias");
-            check(cudaMemcpyAsync(bias[l], W + static_cast<long long>(L.cout_used) * L.cin_used * 9,
-                      L.cout_used * sizeof(float), cudaMemcpyDeviceToDevice, stream), "bias");
+            tasks.push_back({offset[l], L.cout_used, L.cin_used, 0, 0, L.cout, L.cin, nullptr, bias[l]});
         }
-        check(cudaGetLastError(), "pack");
+        pack_tasks = alloc<PackTask>(tasks.size());
+        pack_count = static_cast<int>(tasks.size());
+        cudaMemcpy(pack_tasks, tasks.data(), tasks.size() * sizeof(PackTask), cudaMemcpyHostToDevice);
     }
 
     // one convolution: input x (cin channels) at hh x ww
     void conv(int l, const void* x, int cin, int hh, int ww, const void* wts, const float* b, int cout, int relu, void* y,
-        int ych, int yoff, void* pool = nullptr, int up = 0) {
+        int ych, int yoff, void* pool = nullptr, int up = 0, const void* relu_of = nullptr) {
         CUtensorMap map;
         if (!conv_input_map(&map, x, n, hh, ww, cin)) throw std::string("tensor map");
-        check(launch_conv3x3(map, n, hh, ww, cin, wts, b, cout, relu, y, ych, yoff, err, sms, stream, pool, up), "conv");
+        check(launch_conv3x3(map, n, hh, ww, cin, wts, b, cout, relu, y, ych, yoff, err, sms, stream, pool, up, 0, relu_of),
+            "conv");
         (void)l;
     }
 
@@ -385,35 +381,14 @@ struct Trainer {
             "wgrad");
     }
 
-    // input gradient of layer l: dX (cin channels, written at channel xoff of an xcs tensor) from dz (cout channels)
-    void dgrad(int l, const void* dz, int hh, int ww, void* dx, int xcs, int xoff) {
+    // input gradient of layer l: dX (cin channels, written at channel xoff of an xcs tensor) from dz (cout
+    // channels); with `relu_of`, the layer's input after its ReLU, already masked by that ReLU
+    void dgrad(int l, const void* dz, int hh, int ww, void* dx, int xcs, int xoff, const void* relu_of = nullptr) {
         const LayerSpec& L = kLayers[l];
         for (int k = 0; k * 64 < L.cin; ++k) {
             const int oc = L.cin - 64 * k < 64 ? L.cin - 64 * k : 64;
-            conv(l, dz, L.cout, hh, ww, wb[l][k], zero_bias, oc, 0, dx, xcs, xoff + 64 * k);
+            conv(l, dz, L.cout, hh, ww, wb[l][k], zero_bias, oc, 0, dx, xcs, xoff + 64 * k, nullptr, 0, relu_of);
         }
-    }
-
-    static bool by8(std::initializer_list<int> v) {
-        for (int x : v) {
-            if (x % 8 != 0) return false;
-        }
-        return true;
-    }
-
-    void mask(const void* g, int gcs, int goff, const void* y, int ycs, int yoff, void* out, int ocs, int ooff, int ch,
-        int hh, int ww) {
-        if (by8({gcs, goff, ycs, yoff, ocs, ooff, ch})) {
-            k_relu_mask8<<<grid_of(static_cast<long long>(n) * hh * ww * (ch / 8)), 256, 0, stream>>>(
-                static_cast<const uint4*>(g), gcs / 8, goff / 8, static_cast<const uint4*>(y), ycs / 8, yoff / 8,
-                static_cast<uint4*>(out), ocs / 8, ooff / 8, ch / 8, n, hh * ww);
-            check(cudaGetLastError(), "mask");
-            return;
-        }
-        k_relu_mask<<<grid_of(static_cast<long long>(n) * hh * ww * ch), 256, 0, stream>>>(
-            static_cast<const __nv_bfloat16*>(g), gcs, goff, static_cast<const __nv_bfloat16*>(y), ycs, yoff,
-            static_cast<__nv_bfloat16*>(out), ocs, ooff, ch, n, hh, ww);
-        check(cudaGetLastError(), "mask");
     }
 
     void backward(const void* in16) {
@@ -421,12 +396,10 @@ struct Trainer {
         const long long full = static_cast<long long>(n) * h * w, half = full / 4, quarter = full / 16;
         // head (no ReLU): dZ = loss gradient
         wgrad(10, t6, h, w, g_out16);
-        dgrad(10, g_out16, h, w, g_t6, 32, 0);
+        dgrad(10, g_out16, h, w, g_t6, 32, 0, t6);
         // d1b, d1a
-        mask(g_t6, 32, 0, t6, 32, 0, g_t6, 32, 0, 32, h, w);
         wgrad(9, t5, h, w, g_t6);
-        dgrad(9, g_t6, h, w, g_t5, 32, 0);
-        mask(g_t5, 32, 0, t5, 32, 0, g_t5, 32, 0, 32, h, w);
+        dgrad(9, g_t6, h, w, g_t5, 32, 0, t5);
         wgrad(8, cat1, h, w, g_t5);
         dgrad(8, g_t5, h, w, g_cat1, 80, 0);
         // d2b: its output was upsampled into cat1[32:80]
@@ -434,9 +407,8 @@ struct Trainer {
             reinterpret_cast<const uint4*>(cat1), 10, 4, reinterpret_cast<uint4*>(g_u7), 6, n, h2, w2);
         check(cudaGetLastError(), "up backward");
         wgrad(7, t4, h2, w2, g_u7);
-        dgrad(7, g_u7, h2, w2, g_t4, 48, 0);
+        dgrad(7, g_u7, h2, w2, g_t4, 48, 0, t4);
         // d2a
-        mask(g_t4, 48, 0, t4, 48, 0, g_t4, 48, 0, 48, h2, w2);
         wgrad(6, cat2, h2, w2, g_t4);
         dgrad(6, g_t4, h2, w2, g_cat2, 112, 0);
         // e3b: its output was upsampled into cat2[48:112]
@@ -444,9 +416,8 @@ struct Trainer {
             reinterpret_cast<const uint4*>(cat2), 14, 6, reinterpret_cast<uint4*>(g_u5), 8, n, h4, w4);
         check(cudaGetLastError(), "up backward");
         wgrad(5, t3, h4, w4, g_u5);
-        dgrad(5, g_u5, h4, w4, g_t3, 64, 0);
+        dgrad(5, g_u5, h4, w4, g_t3, 64, 0, t3);
         // e3a
-        mask(g_t3, 64, 0, t3, 64, 0, g_t3, 64, 0, 64, h4, w4);
         wgrad(4, p2, h4, w4, g_t3);
         dgrad(4, g_t3, h4, w4, g_p2, 48, 0);
         // e2b: output in cat2[0:48] (skip) and pooled into p2
@@ -455,9 +426,8 @@ struct Trainer {
             w2);
         check(cudaGetLastError(), "pool backward");
         wgrad(3, t2, h2, w2, g3);
-        dgrad(3, g3, h2, w2, g_t2, 48, 0);
+        dgrad(3, g3, h2, w2, g_t2, 48, 0, t2);
         // e2a
-        mask(g_t2, 48, 0, t2, 48, 0, g_t2, 48, 0, 48, h2, w2);
         wgrad(2, p1, h2, w2, g_t2);
         dgrad(2, g_t2, h2, w2, g_p1, 32, 0);
         // e1b: output in cat1[0:32] (skip) and pooled into p1
@@ -466,20 +436,18 @@ struct Trainer {
             w);
         check(cudaGetLastError(), "pool backward");
         wgrad(1, t1, h, w, g1);
-        dgrad(1, g1, h, w, g_t1, 32, 0);
+        dgrad(1, g1, h, w, g_t1, 32, 0, t1);
         // e1a (its input needs no gradient)
-        mask(g_t1, 32, 0, t1, 32, 0, g_t1, 32, 0, 32, h, w);
         wgrad(0, in16, h, w, g_t1);
     }
 
     // forward, loss, backward; then Adam when lr > 0. Returns the mean loss.
     float step(const void* in16, const float* target, float lr) {
-        check(cudaMemsetAsync(err, 0, sizeof(int), stream), "err");
-        check(cudaMemsetAsync(loss, 0, sizeof(double), stream), "loss");
+        check(cudaMemsetAsync(loss, 0, 2 * sizeof(double), stream), "loss");
         pack();
         forward(in16);
         const long long full = static_cast<long long>(n) * h * w;
-        k_loss_grad<<<grid_of(full), 256, 0, stream>>>(out16, target, n, h, w, g_out16, loss);
+        k_loss_grad<<<std::min(grid_of(full), 4 * sms), 256, 0, stream>>>(out16, target, full, h * w, g_out16, loss);
         check(cudaGetLastError(), "loss");
         backward(in16);
         if (lr > 0.0f) {
@@ -489,11 +457,12 @@ struct Trainer {
             k_adam<<<grid_of(count), 256, 0, stream>>>(params, grads, m, v, count, lr, 0.9f, 0.999f, 1e-8f, c1, c2);
             check(cudaGetLastError(), "adam");
         }
-        double h_loss = 0.0;
-        int h_err = 0;
-        check(cudaMemcpyAsync(&h_loss, loss, sizeof(double), cudaMemcpyDeviceToHost, stream), "loss");
-        check(cudaMemcpyAsync(&h_err, err, sizeof(int), cudaMemcpyDeviceToHost, stream), "err");
+        double h_result[2] = {0.0, 0.0};
+        check(cudaMemcpyAsync(h_result, loss, sizeof h_result, cudaMemcpyDeviceToHost, stream), "loss");
         check(cudaStreamSynchronize(stream), "step");
+        const double h_loss = h_result[0];
+        int h_err = 0;
+        std::memcpy(&h_err, &h_result[1], sizeof h_err);
         if (h_err != 0) throw std::string("a bounded wait inside a training kernel ran out (code ") + std::to_string(h_err) + ")";
         return static_cast<float>(h_loss / static_cast<double>(full * 3));
     }
