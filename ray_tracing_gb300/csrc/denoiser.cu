@@ -1,4 +1,6 @@
-// Denoiser convolutions on the sm_103a tensor cores.
+// Denoiser convolutions on the sm_103a tensor cores, by tiles: the form narrow
+// images and c_in = 128 with c_out = 64 take (conv_rows_fits); the others run
+// k_conv_rows (conv_rows.cu).
 //
 // k_conv3x3 is an implicit-GEMM 3x3 convolution (stride 1, zero padding 1) over
 // channel-blocked BF16 tensors, [n][c/8][h][w][8] (8 channels innermost, then
@@ -546,7 +548,10 @@ extern "C" rtgb_status rtgb_conv3x3_bf16(const void* x, int32_t n, int32_t h, in
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const cudaError_t e = launch_conv3x3(map, n, h, w, c_in, packed_weight, bias, c_out, relu, y, y_channels,
+    const cudaError_t e = conv_rows_fits(w, c_in, c_out)
+        ? launch_conv_rows(x, n, h, w, c_in, packed_weight, bias, c_out, relu, y, y_channels, y_channel_offset, device_error,
+              sms > 0 ? sms : 1, static_cast<cudaStream_t>(stream), nullptr, 0, nullptr)
+        : launch_conv3x3(map, n, h, w, c_in, packed_weight, bias, c_out, relu, y, y_channels,
         y_channel_offset, device_error, sms > 0 ? sms : 1, static_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) {
         set_message(message, message_size, cudaGetErrorString(e));
@@ -676,6 +681,7 @@ struct Acts {
     __nv_bfloat16 *p1 = nullptr, *t2 = nullptr, *cat2 = nullptr, *t4 = nullptr, *t4b = nullptr;
     __nv_bfloat16 *p2 = nullptr, *t3 = nullptr, *t3b = nullptr;
     CUtensorMap maps[kLayerCount];
+    const void* inputs[kLayerCount] = {};
     int stages[kLayerCount] = {};  // halo stages per layer chosen by unet_tune (0: the conv_stages rule)
     bool tuned = false;
     DevMem scratch_err;            // error flag of the tuning launches
@@ -783,6 +789,7 @@ Acts* unet_buffers(UNet* unet, int n, int h, int w) {
             delete net;
             return nullptr;
         }
+        net->inputs[li] = inputs[li].x;
     }
     net->n = n;
     net->h = h;
@@ -842,6 +849,7 @@ bool unet_tune(UNet* unet, Acts* a) {
     for (int li = 0; li < kLayerCount && ok; ++li) {
         const LayerSpec& l = kLayers[li];
         const LayerCall c = layer_call(a, li, a->h, a->w);
+        if (conv_rows_fits(c.ww, l.cin, l.cout)) continue;  // k_conv_rows has no such choice
         float best = 1e30f;
         int best_s = 0;
         for (int s = 2; s <= kMaxStages; s += 2) {  // even counts: two issuers per CTA
@@ -898,6 +906,10 @@ cudaError_t unet_run(UNet* unet, const FrameParams* fp, long long pixel_offset, 
     const int h2 = (h + 1) / 2, w2 = (w + 1) / 2, h4 = (h2 + 1) / 2, w4 = (w2 + 1) / 2;
     auto conv = [&](int li, int hh, int ww, void* y, int ych, int yoff, void* pool = nullptr, int up = 0) {
         const LayerSpec& l = kLayers[li];
+        if (conv_rows_fits(ww, l.cin, l.cout)) {
+            return launch_conv_rows(net->inputs[li], n, hh, ww, l.cin, unet->weights[li].p,
+                static_cast<const float*>(unet->biases[li].p), l.cout, l.relu, y, ych, yoff, err, sms, stream, pool, up, nullptr);
+        }
         return launch_conv3x3(net->maps[li], n, hh, ww, l.cin, unet->weights[li].p, static_cast<const float*>(unet->biases[li].p),
             l.cout, l.relu, y, ych, yoff, err, sms, stream, pool, up, net->stages[li]);
     };

@@ -55,6 +55,13 @@ cudaError_t conv_init();
 cudaError_t launch_conv3x3(const CUtensorMap& map, int n, int h, int w, int cin, const void* weight, const float* bias,
     int cout, int relu, void* y, int y_channels, int y_offset, int* err, int grid_limit, cudaStream_t stream,
     void* pool = nullptr, int up = 0, int stages = 0, const void* mask = nullptr);
+// The same layer by image rows (conv_rows.cu), the same bits: three taps an
+// instruction. `x` is the input tensor itself.
+cudaError_t launch_conv_rows(const void* x, int n, int h, int w, int cin, const void* weight, const float* bias, int cout,
+    int relu, void* y, int y_channels, int y_offset, int* err, int sms, cudaStream_t stream, void* pool, int up,
+    const void* mask);
+// Whether launch_conv_rows takes (and is the faster for) a width and channel counts.
+bool conv_rows_fits(int w, int cin, int cout);
 // Weight (cout_used x cin_used x 3 x 3, FP32) and bias gradients of a k_conv3x3
 // layer (denoiser_train.cu); `partial` holds wgrad_partial_bytes of at least
 // min(sms, tiles) CTAs.

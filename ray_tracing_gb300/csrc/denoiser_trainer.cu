@@ -350,6 +350,11 @@ struct Trainer {
     // one convolution: input x (cin channels) at hh x ww
     void conv(int l, const void* x, int cin, int hh, int ww, const void* wts, const float* b, int cout, int relu, void* y,
         int ych, int yoff, void* pool = nullptr, int up = 0, const void* relu_of = nullptr) {
+        if (conv_rows_fits(ww, cin, cout)) {
+            check(launch_conv_rows(x, n, hh, ww, cin, wts, b, cout, relu, y, ych, yoff, err, sms, stream, pool, up, relu_of),
+                "conv");
+            return;
+        }
         CUtensorMap map;
         if (!conv_input_map(&map, x, n, hh, ww, cin)) throw std::string("tensor map");
         check(launch_conv3x3(map, n, hh, ww, cin, wts, b, cout, relu, y, ych, yoff, err, sms, stream, pool, up, 0, relu_of),
