@@ -441,11 +441,23 @@ struct PackedLight {
 // One leaf-ordered primitive record, 64 bytes (four float4):
 //   sphere:   [0] center.xyz radius
 //   quad:     [0] origin.xyz n.x  [1] edge_u.xyz n.y  [2] edge_v.xyz n.z  [3] w.xyz
-//   triangle: [0] p0.xyz          [1] e1.xyz          [2] e2.xyz
+//   triangle: [0] p0.xyz material [1] e1.xyz flags    [2] e2.xyz
+//   (material as int bits, also in a sphere's [1].w; flags: kTriNormals, kTriTexcoords)
 // [3].w always holds the primitive code (type << 28 | index) as int bits.
 // n = unit quad normal and w = n / |n|^2 are computed on the host with the
 // reference's float operations (programs.cu:1451-1476), e1/e2 = p1-p0, p2-p0.
+// The shading kernels rebuild a hit from the same record (the trace leaves its
+// slot), four aligned 16-byte loads where the authored 108-byte triangle took 27
+// scattered 4-byte ones.
 struct PrimRecord {
+    float4 q[4];
+};
+constexpr int kTriNormals = 1;
+constexpr int kTriTexcoords = 2;
+
+// A triangle's vertex normals and texture coordinates beside its leaf record,
+// 64 bytes: [0] n0.xyz uv0.x  [1] n1.xyz uv0.y  [2] n2.xyz uv1.x  [3] uv1.y uv2.xy -
+struct TriAttr {
     float4 q[4];
 };
 
@@ -471,6 +483,7 @@ constexpr int kStagedNodes4 = 64;         // BVH4 nodes the trace kernels keep i
 
 struct DeviceScene {
     const PrimRecord* prims;      // leaf order
+    const TriAttr* tri_attr;      // leaf order (read where a triangle's flags say so), null without triangles
     const BvhNode* nodes;         // binary LBVH (build, refit, parity downloads)
     int prim_count;
     int node_count;
@@ -487,6 +500,7 @@ struct DeviceScene {
     const PackedLight* lights;
     const float* light_cdf;
     const int* light_guide;       // kGuide + 1 bucket starts over light_cdf (sample_cdf_guided)
+    const float4* light_tri;      // 3 per light, of triangle lights: p0 material, p1 (1 with texture coordinates), p2
     int light_count;
     int environment_light;        // index into lights or -1
     const int* sphere_light;       // primitive -> light index or -1
@@ -861,12 +875,14 @@ RTGB_D void order_keys(unsigned& a, unsigned& b) {
 // an insertion sort took 27.3 / 20.7 ms of trace / shadow per frame of the
 // 4 M-triangle room, this 23.3 / 18.3 ms (the 1 M-triangle terrain's trace 3.37
 // -> 2.82 ms). Refilling finished lanes with the next ray inside the loop was
-// slower at every threshold (the terrain's trace 3.6-5.0 ms). Returns the code or -1.
+// slower at every threshold (the terrain's trace 3.6-5.0 ms). Returns the code or
+// -1 and leaves the leaf slot in `best_slot`.
 // `overflow` counts subtrees dropped by a full stack (never silently).
 // `staged` / `staged_count`: a shared-memory copy of the first nodes (or null / 0).
 RTGB_D int traverse_closest(const DeviceScene& s, const float3& o, const float3& d, float tmin, float& closest,
-    int& overflow, const float4* staged = nullptr, int staged_count = 0) {
+    int& best_slot, int& overflow, const float4* staged = nullptr, int staged_count = 0) {
     int best = -1;
+    best_slot = 0;
     if (s.prim_count <= 0) return -1;
     if (s.prim_count == 1) {
         const PrimRecord p = load_prim(s.prims, 0);
@@ -891,11 +907,13 @@ RTGB_D int traverse_closest(const DeviceScene& s, const float3& o, const float3&
 #pragma unroll
         for (int k = 0; k < 4; ++k) leaves |= child[k] < 0 ? hit & (1u << k) : 0u;
         for (unsigned m = leaves; m != 0; m &= m - 1) {
-            const PrimRecord p = load_prim(s.prims, ~pick4(child, __ffs(m) - 1));
+            const int slot = ~pick4(child, __ffs(m) - 1);
+            const PrimRecord p = load_prim(s.prims, slot);
             float t;
             if (prim_hit(p, o, d, tmin, closest, t)) {
                 closest = t;
                 best = prim_code(p);
+                best_slot = slot;
             }
         }
         unsigned key[4];

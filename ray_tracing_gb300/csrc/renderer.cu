@@ -39,7 +39,7 @@ __global__ void k_prim_records(DeviceScene s, PrimRecord* records, float4* aabb_
             const float3 c = ld3(sp.center);
             const float rr = fabsf(sp.radius);
             r.q[0] = make_float4(c.x, c.y, c.z, sp.radius);
-            r.q[1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            r.q[1] = make_float4(0.0f, 0.0f, 0.0f, __int_as_float(sp.material_index));
             r.q[2] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             lo = f3(c.x - rr, c.y - rr, c.z - rr);
             hi = f3(c.x + rr, c.y + rr, c.z + rr);
@@ -71,8 +71,9 @@ __global__ void k_prim_records(DeviceScene s, PrimRecord* records, float4* aabb_
             const rtgb_triangle t = s.triangles[k];
             const float3 p0 = ld3(t.p0), p1 = ld3(t.p1), p2 = ld3(t.p2);
             const float3 e1 = sub(p1, p0), e2 = sub(p2, p0);
-            r.q[0] = make_float4(p0.x, p0.y, p0.z, 0.0f);
-            r.q[1] = make_float4(e1.x, e1.y, e1.z, 0.0f);
+            const int flags = (t.has_vertex_normals != 0 ? kTriNormals : 0) | (t.has_texcoords != 0 ? kTriTexcoords : 0);
+            r.q[0] = make_float4(p0.x, p0.y, p0.z, __int_as_float(t.material_index));
+            r.q[1] = make_float4(e1.x, e1.y, e1.z, __int_as_float(flags));
             r.q[2] = make_float4(e2.x, e2.y, e2.z, 0.0f);
             r.q[3] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             lo = f3(fminf(fminf(p0.x, p1.x), p2.x), fminf(fminf(p0.y, p1.y), p2.y), fminf(fminf(p0.z, p1.z), p2.z));
@@ -86,9 +87,19 @@ __global__ void k_prim_records(DeviceScene s, PrimRecord* records, float4* aabb_
     }
 }
 
-__global__ void k_gather_records(const PrimRecord* __restrict__ in, const int* __restrict__ order, PrimRecord* out,
-    int n) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) out[i] = in[order[i]];
+__global__ void k_gather_records(const rtgb_triangle* __restrict__ triangles, const PrimRecord* __restrict__ in,
+    const int* __restrict__ order, PrimRecord* out, TriAttr* attr, int n) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const PrimRecord r = in[order != nullptr ? order[i] : 0];
+        out[i] = r;
+        const int code = prim_code(r);
+        if (attr == nullptr || static_cast<unsigned>(code) >> 28 != 2 || __float_as_int(r.q[1].w) == 0) continue;
+        const rtgb_triangle& t = triangles[code & 0x0fffffff];
+        attr[i].q[0] = make_float4(t.n0[0], t.n0[1], t.n0[2], t.uv0[0]);
+        attr[i].q[1] = make_float4(t.n1[0], t.n1[1], t.n1[2], t.uv0[1]);
+        attr[i].q[2] = make_float4(t.n2[0], t.n2[1], t.n2[2], t.uv1[0]);
+        attr[i].q[3] = make_float4(t.uv1[1], t.uv2[0], t.uv2[1], 0.0f);
+    }
 }
 
 void launch_prim_records(const DeviceScene& scene, PrimRecord* records, float4* aabb_lo, float4* aabb_hi, float pad,
@@ -97,8 +108,9 @@ void launch_prim_records(const DeviceScene& scene, PrimRecord* records, float4* 
     k_prim_records<<<std::min((n + 255) / 256, 8192), 256, 0, stream>>>(scene, records, aabb_lo, aabb_hi, pad);
 }
 
-void launch_gather_records(const PrimRecord* in, const int* order, PrimRecord* out, int n, cudaStream_t stream) {
-    k_gather_records<<<std::min((n + 255) / 256, 8192), 256, 0, stream>>>(in, order, out, n);
+void launch_gather_records(const DeviceScene& scene, const PrimRecord* in, const int* order, PrimRecord* out, TriAttr* attr,
+    int n, cudaStream_t stream) {
+    k_gather_records<<<std::min((n + 255) / 256, 8192), 256, 0, stream>>>(scene.triangles, in, order, out, attr, n);
 }
 
 namespace {
@@ -209,11 +221,12 @@ struct rtgb_renderer {
     float last_denoise_ms = 0.0f;
     cudaEvent_t ev_dn0 = nullptr, ev_dn1 = nullptr;
     DevBuf light_guide, analytic_guide;  // CDF guide tables of the NEE searches (sample_cdf_guided)
+    DevBuf light_tri;                    // triangle lights' hot records (DeviceScene::light_tri)
     DevBuf material_lum, light_counts;   // light table inputs; its counts (+ the LBVH scale word)
     // device copy of an instanced mesh set (rtgb_prepare_scene_instanced, mesh_flatten.cu)
     DevBuf mesh_points, mesh_corners, mesh_normals, mesh_texcoords, mesh_materials, mesh_protos, mesh_insts;
     DevBuf spheres, quads, triangles, media, materials, textures, texels, lights, light_cdf, sphere_light, quad_light,
-        triangle_light, analytic, analytic_cdf, analytic_nodes, analytic_leaf, infinite_analytic, prims, nodes,
+        triangle_light, analytic, analytic_cdf, analytic_nodes, analytic_leaf, infinite_analytic, prims, tri_attr, nodes,
         sorted_keys, sorted_vals;
     int prim_count = 0;
     int analytic_bvh_count = 0;
@@ -277,6 +290,7 @@ struct rtgb_renderer {
     cudaEvent_t ev_copied[2]{};            // last copy enqueued from frames[slot]
     cudaEvent_t ev_older_copied = nullptr; // every copy of frames before the latest downloaded one
     bool copy_pending[2] = {false, false};
+    long long zero_reservoirs[2] = {0, 0};  // leading pixels of frames[slot] whose reservoir records are zero
     uint64_t frame_serial = 0;             // frames rendered
     uint64_t download_serial = 0;          // frame_serial of the frame last downloaded asynchronously
     bool stage_timing = false;
@@ -339,10 +353,10 @@ struct rtgb_renderer {
         if (copy_stream) cudaStreamDestroy(copy_stream);
         DevBuf* bufs[] = {&spheres, &quads, &triangles, &media, &materials, &textures, &texels, &lights, &light_cdf,
             &sphere_light, &quad_light, &triangle_light, &analytic, &analytic_cdf, &analytic_nodes, &analytic_leaf,
-            &infinite_analytic, &prims, &nodes, &sorted_keys, &sorted_vals, &frame_mem[0], &frame_mem[1], &path_mem,
+            &infinite_analytic, &prims, &tri_attr, &nodes, &sorted_keys, &sorted_vals, &frame_mem[0], &frame_mem[1], &path_mem,
             &counters_mem, &fp_mem, &debug_rgba, &openpbr, &analytic_hot, &bvh_children, &bvh_parent, &nodes4, &child4, &ref4,
             &light_guide, &analytic_guide, &material_lum, &light_counts, &mesh_points, &mesh_corners, &mesh_normals,
-            &mesh_texcoords, &mesh_materials, &mesh_protos, &mesh_insts, &lbvh_mem, &collapse_mem, &unsorted, &light_mem};
+            &mesh_texcoords, &mesh_materials, &mesh_protos, &mesh_insts, &light_tri, &lbvh_mem, &collapse_mem, &unsorted, &light_mem};
         for (DevBuf* b : bufs) b->release();
         for (auto& slot : cam_res) {
             for (auto& r : slot) {
@@ -764,6 +778,9 @@ struct rtgb_renderer {
             d.sphere_light = lt.sphere_light;
             d.quad_light = lt.quad_light;
             d.triangle_light = lt.triangle_light;
+            d.light_tri = static_cast<const float4*>(light_tri.ensure(std::max<size_t>(static_cast<size_t>(d.light_count), 1) * 3 * sizeof(float4)));
+            launch_light_tri(d, const_cast<float4*>(d.light_tri), stream);
+            RTGB_CHECK(cudaGetLastError());
         }
 
         // analytic lights: CDF array, infinite list and a BVH over finite ones
@@ -819,13 +836,17 @@ struct rtgb_renderer {
         unsorted.ensure(static_cast<size_t>(n) * sizeof(PrimRecord));
         LbvhScratch ls = lbvh_carve(lbvh_mem.ensure(lbvh_scratch_bytes(n)), n);
         PrimRecord* recs = static_cast<PrimRecord*>(prims.ensure(static_cast<size_t>(n) * sizeof(PrimRecord)));
+        TriAttr* attr = d.triangle_count > 0
+                            ? static_cast<TriAttr*>(tri_attr.ensure(static_cast<size_t>(n) * sizeof(TriAttr)))
+                            : nullptr;
+        d.tri_attr = attr;
         launch_prim_records(d, unsorted.as<PrimRecord>(), ls.aabb_lo, ls.aabb_hi, pad, stream);
         RTGB_CHECK(cudaGetLastError());
         if (n >= 2 && kind == 2) {
             // same counts: the kept leaf order and hierarchy, boxes refitted bottom-up
             BvhNode* nd = nodes.as<BvhNode>();
             RTGB_CHECK(lbvh_refit(ls, n, sorted_vals.as<int>(), bvh_children.as<int>(), bvh_parent.as<int>(), nd, stream));
-            launch_gather_records(unsorted.as<PrimRecord>(), sorted_vals.as<int>(), recs, n, stream);
+            launch_gather_records(d, unsorted.as<PrimRecord>(), sorted_vals.as<int>(), recs, attr, n, stream);
             RTGB_CHECK(cudaGetLastError());
             RTGB_CHECK(fill_bvh4(nd, child4.as<int>(), ref4.as<int>(), node4_count, nodes4.as<float4>(), stream));
             d.nodes = nd;
@@ -835,7 +856,7 @@ struct rtgb_renderer {
             int* svals = nullptr;
             uint32_t* skeys = nullptr;
             RTGB_CHECK(lbvh_build(ls, n, nd, &svals, &skeys, stream));
-            launch_gather_records(unsorted.as<PrimRecord>(), svals, recs, n, stream);
+            launch_gather_records(d, unsorted.as<PrimRecord>(), svals, recs, attr, n, stream);
             RTGB_CHECK(cudaGetLastError());
             sorted_keys.ensure(static_cast<size_t>(n) * sizeof(uint32_t));
             sorted_vals.ensure(static_cast<size_t>(n) * sizeof(int));
@@ -861,7 +882,8 @@ struct rtgb_renderer {
             d.nodes = nd;
             d.node_count = n - 1;
         } else {
-            RTGB_CHECK(cudaMemcpyAsync(recs, unsorted.p, sizeof(PrimRecord), cudaMemcpyDeviceToDevice, stream));
+            launch_gather_records(d, unsorted.as<PrimRecord>(), nullptr, recs, attr, n, stream);
+            RTGB_CHECK(cudaGetLastError());
             d.nodes = nullptr;
             d.node_count = 0;
             node4_count = 0;
@@ -960,6 +982,7 @@ struct rtgb_renderer {
             // asynchronous downloads may still read the old buffers
             if (copy_stream) RTGB_CHECK(cudaStreamSynchronize(copy_stream));
             copy_pending[f] = false;
+            zero_reservoirs[f] = 0;
             char* p = static_cast<char*>(frame_mem[f].ensure(static_cast<size_t>(pixels) * per + 2304));
             auto take = [&](size_t bytes) {
                 char* r = p;
@@ -1273,6 +1296,8 @@ struct rtgb_renderer {
         const bool bucket = shade_order > 0 ||
             (shade_order == 0 && (scene.openpbr_count > 0 || scene.material_count > kBucketMaterials));
         fp.sort_from_bounce = !bucket ? INT_MAX : (shade_order == 1 ? 1 : 0);
+        fp.openpbr = scene.openpbr_count > 0 ? 1 : 0;
+        fp.zero_reservoirs = fp.restir_enabled != 0 || total_pixels > zero_reservoirs[cur] ? 1 : 0;
         fp.cur = frames[cur];
         fp.hist = frames[cur ^ 1];
         // Pageable source: the copy is staged before the call returns, so the
@@ -1316,6 +1341,7 @@ struct rtgb_renderer {
             last_w[c] = rig.cameras[c].width;
             last_h[c] = rig.cameras[c].height;
         }
+        zero_reservoirs[cur] = fp.restir_enabled != 0 ? 0 : std::max(zero_reservoirs[cur], total_pixels);
         last_count = active;
         last_denoised = denoise_this_frame;
         last_spp = spp;

@@ -16,14 +16,14 @@ void launch_shade_pbr(const FrameParams* fp, DeviceScene scene, Paths paths, Cou
 
 LaunchShape query_shade_pbr_shape(int sm_count) {
     int blocks = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_shade<true, true>, 128, 0);
-    return LaunchShape{sm_count * (blocks > 0 ? blocks : 1), 128};
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_shade<true, true>, kPbrBlock, 0);
+    return LaunchShape{sm_count * (blocks > 0 ? blocks : 1), kPbrBlock};
 }
 
 LaunchShape query_scatter_pbr_shape(int sm_count) {
     int blocks = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_scatter<true>, 128, 0);
-    return LaunchShape{sm_count * (blocks > 0 ? blocks : 1), 128};
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_scatter<true>, kPbrBlock, 0);
+    return LaunchShape{sm_count * (blocks > 0 ? blocks : 1), kPbrBlock};
 }
 
 }  // namespace rtgb

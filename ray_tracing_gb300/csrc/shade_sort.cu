@@ -29,13 +29,14 @@ __device__ __forceinline__ int shade_key(const DeviceScene& s, const float4& hr)
     if (code == -1) return 0;
     const int type = static_cast<int>(static_cast<unsigned>(code) >> 28);
     const int idx = code & 0x0fffffff;
+    const PrimRecord* rec = s.prims + __float_as_int(hr.w);  // of the leaf the trace hit
     int mi;
     if (type == 0) {
-        mi = __ldg(&s.spheres[idx].material_index);
+        mi = __float_as_int(__ldg(&rec->q[1].w));
     } else if (type == 1) {
         mi = __ldg(&s.quads[idx].material_index);
     } else if (type == 2) {
-        mi = __ldg(&s.triangles[idx].material_index);
+        mi = __float_as_int(__ldg(&rec->q[0].w));
     } else {
         return 1;
     }

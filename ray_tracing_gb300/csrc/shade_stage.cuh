@@ -17,6 +17,12 @@ namespace rtgb {
 namespace {
 constexpr int kFlagValid = 1;
 constexpr int kFlagDelta = 2;
+// Threads of a block of the OpenPBR shade kernels, started together for every
+// path (a barrier an iteration): warps that walk the same long code at the same
+// time share its instruction fetches. Against 128 threads without barriers the
+// 1 M-triangle terrain's first shade stage takes 1.31 instead of 1.51 ms and the
+// gallery's frame 4.91 instead of 5.08; 384 threads measure the same, 768 worse.
+constexpr int kPbrBlock = 256;
 
 RTGB_D int camera_of_path(const FrameParams& fp, long long path) {
     int c = 0;
@@ -176,7 +182,8 @@ RTGB_D bool previous_pixel(const FrameParams& fp, int c, const Hit& h, int& inde
 // restir_target_at_previous_surface, programs.cu:2210-2247: one closest-hit
 // visibility ray from the previous camera to the reuse source's surface.
 template <bool kPbr>
-RTGB_D float target_at_previous(ShadeCtx& ctx, int c, const Surface& src, const Candidate& sel, bool bsdf_avail) {
+RTGB_D float target_at_previous(ShadeCtx& ctx, int c, const Surface& src, const Candidate& sel, bool bsdf_avail,
+    pbr::Mat& spm) {
     const FrameParams& fp = ctx.fp;
     if (fp.prev_valid[c] == 0) return 0.0f;
     const float3 spos = ld3(src.position);
@@ -187,10 +194,11 @@ RTGB_D float target_at_previous(ShadeCtx& ctx, int c, const Surface& src, const 
     const float3 dir = mul(off, 1.0f / dist);
     float closest = dist + 0.05f;
     ++ctx.vis_rays;
-    const int code = traverse_closest(ctx.s, origin, dir, kRayEpsilon, closest, ctx.overflow);
+    int slot;
+    const int code = traverse_closest(ctx.s, origin, dir, kRayEpsilon, closest, slot, ctx.overflow);
     if (code == -1) return 0.0f;
     Hit sh;
-    if (!reconstruct_surface<kPbr>(ctx.s, code, origin, dir, sh)) return 0.0f;
+    if (!reconstruct_surface<kPbr>(ctx.s, code, slot, origin, dir, sh)) return 0.0f;
     if (sh.mtype != src.material_type || sh.ptype != src.primitive_type || sh.pidx != src.primitive_index) {
         return 0.0f;
     }
@@ -198,7 +206,6 @@ RTGB_D float target_at_previous(ShadeCtx& ctx, int c, const Surface& src, const 
     if (len_sq(sub(sh.pos, spos)) > tol * tol || dot(sh.sn, ld3(src.normal)) < 0.95f) return 0.0f;
     const LightSample l = restir_candidate<kPbr>(ctx, sh.pos, sh.sn, sh.mtype, sel.light_index, sel.u0, sel.u1);
     // the source path state is fresh: unit throughput, ray from the previous camera
-    pbr::Mat spm;
     if constexpr (kPbr) {
         if (sh.mtype == 5) openpbr_scattering(ctx.s, sh, spm);
     }
@@ -209,6 +216,9 @@ RTGB_D float target_at_previous(ShadeCtx& ctx, int c, const Surface& src, const 
 
 // The surface of a stored reservoir (its first sector).
 RTGB_D Surface load_surface(const ReservoirRec* r) { return unpack_surface(r->q[0], r->q[1]); }
+
+// Whether paths park their reservoirs in Paths::res_scratch (several samples a pixel).
+RTGB_D bool scratch_reservoirs(const FrameParams& fp) { return fp.restir_enabled != 0 && fp.spp != 1; }
 
 // Where a bounce-0 path's reservoir lives during the frame: in its pixel's
 // frame record when there is one sample per pixel (written by k_restir_ris,
@@ -237,21 +247,6 @@ RTGB_D ReservoirRec* reservoir_slot(const FrameParams& fp, const Paths& P, const
 // own register budget and occupancy; no value or draw order changes.
 
 constexpr int kMaxSources = kMaxReuseSources;
-// Builds guide[0..kGuide] over cdf (all threads of the block; ends with a barrier).
-RTGB_D void build_guide(const float* cdf, int count, int* guide) {
-    for (int j = threadIdx.x; j <= kGuide; j += blockDim.x) {
-        const float t = static_cast<float>(j) * (1.0f / static_cast<float>(kGuide));
-        int lo = 0, hi = count;
-        while (lo < hi) {
-            const int mid = (lo + hi) >> 1;
-            if (t < cdf[mid]) hi = mid;
-            else lo = mid + 1;
-        }
-        guide[j] = j == kGuide ? count : lo;
-    }
-    __syncthreads();
-}
-
 // meta word of a parked reservoir: source count, selected source + 1, canonical M
 RTGB_D int pack_meta(int nsrc, int selected_src, int canonical) {
     return nsrc | ((selected_src + 1) << 8) | (canonical << 16);
@@ -407,10 +402,11 @@ RTGB_D void restir_finish(ShadeCtx& ctx, const Paths& P, ReservoirRec* slot, lon
 // record and radiance: for the ReSTIR passes, which rebuild the hit and (in
 // k_restir) scatter, and scatter rewrites every previous-scatter field before
 // store_path writes them.
-RTGB_D void load_ray(const Paths& P, int path, PathRegs& st) {
+// `first`: bounce 0, where the throughput is one and not stored yet.
+RTGB_D void load_ray(const Paths& P, int path, bool first, PathRegs& st) {
     st.o = xyz(P.ray_o[path]);
     st.d = xyz(P.ray_d[path]);
-    const float4 thr4 = P.thr[path];
+    const float4 thr4 = first ? make_float4(1.0f, 1.0f, 1.0f, 0.0f) : P.thr[path];
     st.thr = xyz(thr4);
     st.prev_pdf = thr4.w;
     st.rad = f3(0.0f, 0.0f, 0.0f);
@@ -422,6 +418,13 @@ RTGB_D void load_ray(const Paths& P, int path, PathRegs& st) {
     st.prev_ptype = -1;
     st.prev_pidx = -1;
     st.alive = true;
+}
+
+// The state k_shade starts bounce 0 from (trace_primary_ray, programs.cu:2086-2099).
+RTGB_D void load_first(const Paths& P, int path, PathRegs& st) {
+    load_ray(P, path, true, st);
+    st.prev_nrm = f3(0.0f, 0.0f, 1.0f);
+    st.prev_delta = true;
 }
 
 RTGB_D void load_path(const Paths& P, int path, PathRegs& st) {
@@ -553,7 +556,7 @@ RTGB_D bool rebuild_hit(const DeviceScene& s, const float4& hr, const PathRegs& 
         reconstruct_medium<kPbr>(s, code & 0x0fffffff, hr.x, st.o, st.d, h);
         return true;
     }
-    return reconstruct_surface<kPbr>(s, code, st.o, st.d, h);
+    return reconstruct_surface<kPbr>(s, code, __float_as_int(hr.w), st.o, st.d, h);
 }
 
 // The path enters or leaves an OpenPBR random-walk medium (sample_bsdf,
@@ -611,7 +614,7 @@ RTGB_D int subsurface_step(const Paths& P, int path, int sss, const Hit& h, uint
 // against 1.54 at four or five blocks, the 1280 x 720 final room 2.28 against
 // 2.47 / 2.35 ms.
 template <bool kPbr, bool kSplit = false>
-__global__ void __launch_bounds__(128, 6) k_shade(const FrameParams* __restrict__ fpp, DeviceScene s, Paths P,
+__global__ void __launch_bounds__(kSplit ? kPbrBlock : 128, kSplit ? 768 / kPbrBlock : 6) k_shade(const FrameParams* __restrict__ fpp, DeviceScene s, Paths P,
     Counters* counters, int bounce) {
     const FrameParams& fp = *fpp;
     const int in = bounce & 1;
@@ -620,13 +623,19 @@ __global__ void __launch_bounds__(128, 6) k_shade(const FrameParams* __restrict_
     QueueLengths* const filled = &counters->lengths[bounce + 1];
     const bool restir_bounce = fp.restir_enabled != 0 && bounce == 0;
     const int* __restrict__ order = bounce >= fp.sort_from_bounce ? P.sorted : P.queue[in];
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
+    for (int first = blockIdx.x * blockDim.x; first < count; first += gridDim.x * blockDim.x) {
+        if constexpr (kSplit) __syncthreads();
+        const int i = first + static_cast<int>(threadIdx.x);
+        if (i >= count) continue;
         const int path = order[i];
         const float4 hr = P.hit[path];
         const int code = __float_as_int(hr.y);
         const int alight = __float_as_int(hr.z);
         PathRegs st;
-        load_path(P, path, st);
+        if (bounce == 0) load_first(P, path, st);
+        else load_path(P, path, st);
+        const float3 rad_in = st.rad;
+        bool aux = false;
         uint32_t rng = P.rng[path];
         if (fp.record_paths) {
             P.codes[static_cast<long long>(path) * fp.max_bounces + bounce] =
@@ -656,7 +665,7 @@ __global__ void __launch_bounds__(128, 6) k_shade(const FrameParams* __restrict_
             } else {
                 int walk = 0;
                 if constexpr (kPbr) {
-                    const int sss = P.sss_mat[path];
+                    const int sss = bounce == 0 ? -1 : P.sss_mat[path];
                     if (sss >= 0) {
                         walk = subsurface_step(P, path, sss, h, rng, st);
                         thr_changed = true;
@@ -668,7 +677,7 @@ __global__ void __launch_bounds__(128, 6) k_shade(const FrameParams* __restrict_
                 } else if (walk == 0) {
                     // shared, not stack: as in k_scatter (one slot for the
                     // legacy instances, which never touch it)
-                    __shared__ pbr::Mat shade_mats[kPbr ? 128 : 1];
+                    __shared__ pbr::Mat shade_mats[kPbr ? kPbrBlock : 1];
                     pbr::Mat& pm = shade_mats[kPbr ? threadIdx.x : 0];
                     if constexpr (kPbr) {
                         if (h.mtype == 5) openpbr_scattering(s, h, pm);
@@ -676,6 +685,7 @@ __global__ void __launch_bounds__(128, 6) k_shade(const FrameParams* __restrict_
                     if (bounce == 0) {
                         P.aux_n[path] = f4(h.sn, h.t);
                         P.aux_a[path] = f4(h.base, 1.0f);
+                        aux = true;
                     }
                     const float ew = emission_mis_weight(s, st, &h, false);
                     st.rad = add(st.rad, mul(st.thr, mul(h.emis, ew)));
@@ -744,7 +754,8 @@ __global__ void __launch_bounds__(128, 6) k_shade(const FrameParams* __restrict_
                 }
             }
         }
-        P.rad[path] = f4(st.rad, 0.0f);
+        if (bounce == 0 && !aux) P.aux_a[path] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);  // nothing captured
+        if (bounce == 0 || st.rad.x != rad_in.x || st.rad.y != rad_in.y || st.rad.z != rad_in.z) P.rad[path] = f4(st.rad, 0.0f);
         P.rng[path] = rng;
         if (keep) store_path(P, path, st);
         bool any_shadow = false;
@@ -784,17 +795,20 @@ __global__ void __launch_bounds__(128, 6) k_shade(const FrameParams* __restrict_
 // apply_russian_roulette, :1764-1771) of the paths k_shade<kPbr, true> queued,
 // continuing their RNG stream where the next-event estimation left it.
 template <bool kPbr>
-__global__ void __launch_bounds__(128, 6) k_scatter(const FrameParams* __restrict__ fpp, DeviceScene s, Paths P,
+__global__ void __launch_bounds__(kPbrBlock, 768 / kPbrBlock) k_scatter(const FrameParams* __restrict__ fpp, DeviceScene s, Paths P,
     Counters* counters, int bounce) {
     const FrameParams& fp = *fpp;
     const int out = (bounce & 1) ^ 1;
     QueueLengths* const filled = &counters->lengths[bounce + 1];
     const int count = filled->scatter;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
+    for (int first = blockIdx.x * blockDim.x; first < count; first += gridDim.x * blockDim.x) {
+        __syncthreads();
+        const int i = first + static_cast<int>(threadIdx.x);
+        if (i >= count) continue;
         const int path = P.scatter_queue[i];
         const float4 hr = P.hit[path];
         PathRegs st;
-        load_ray(P, path, st);
+        load_ray(P, path, bounce == 0, st);
         uint32_t rng = P.rng[path];
         Hit h;
         rebuild_hit<kPbr>(s, hr, st, h);  // rebuilt in k_shade from the same record
@@ -802,7 +816,7 @@ __global__ void __launch_bounds__(128, 6) k_scatter(const FrameParams* __restric
         // sampler is an out-of-line call that reads them by reference, and on
         // the stack they would travel through L1 / L2 with every other
         // thread's stack (204 B a thread, an odd word stride: no bank conflicts).
-        __shared__ pbr::Mat mats[128];
+        __shared__ pbr::Mat mats[kPbrBlock];
         pbr::Mat& pm = mats[threadIdx.x];
         if constexpr (kPbr) {
             if (h.mtype == 5) openpbr_scattering(s, h, pm);
@@ -821,38 +835,43 @@ __global__ void __launch_bounds__(128, 6) k_scatter(const FrameParams* __restric
 
 // ReSTIR DI for the deferred bounce-0 surfaces: the three passes described at
 // restir_gather, then the BSDF scatter.
-constexpr int kSharedCdf = 4096;
 
-// Shared-memory copy of the analytic-light CDF (when it fits) and its guide table.
+// Shared-memory copy of the candidates' light CDF (when it fits; OpenPBR blocks
+// keep their material blocks there too) and of its guide table.
+template <bool kPbr>
 struct RestirShared {
-    float cdf[kSharedCdf];
+    static constexpr int kCdf = kPbr ? 1024 : 4096;
+    float cdf[kCdf];
     int guide[kGuide + 1];
 };
 
-RTGB_D const float* stage_cdf(const FrameParams& fp, const DeviceScene& s, RestirShared& sh, int& count) {
+template <bool kPbr>
+RTGB_D const float* stage_cdf(const FrameParams& fp, const DeviceScene& s, RestirShared<kPbr>& sh, int& count) {
     const float* src = fp.restir_emissive != 0 ? s.light_cdf : s.analytic_cdf;
+    const int* guide = fp.restir_emissive != 0 ? s.light_guide : s.analytic_guide;
     count = fp.restir_emissive != 0 ? s.light_count : s.analytic_count;
-    const bool shared = count <= kSharedCdf;
-    if (shared) {
-        for (int k = threadIdx.x; k < count; k += blockDim.x) sh.cdf[k] = src[k];
-        __syncthreads();
-    }
-    const float* cdf = shared ? sh.cdf : src;
-    build_guide(cdf, count, sh.guide);
-    return cdf;
+    const bool shared = count <= RestirShared<kPbr>::kCdf;
+    for (int k = threadIdx.x; shared && k < count; k += blockDim.x) sh.cdf[k] = src[k];
+    for (int j = threadIdx.x; j <= kGuide; j += blockDim.x) sh.guide[j] = guide[j];
+    __syncthreads();
+    return shared ? sh.cdf : src;
 }
 
-// Six resident blocks (80 registers) measured fastest among 1, 6, 8 and 10.
+// Six resident blocks (80 registers) measured fastest among 1, 6, 8 and 10 for
+// legacy materials; the OpenPBR instance, whose evaluation calls spill, takes
+// four (128 registers): the 24-light OpenPBR gallery's ReSTIR bounce 2.15 ms
+// against 2.26 at six and 2.24 at three.
 template <bool kPbr>
-__global__ void __launch_bounds__(128, 6) k_restir_ris(const FrameParams* __restrict__ fpp, DeviceScene s, Paths P,
+__global__ void __launch_bounds__(128, kPbr ? 4 : 6) k_restir_ris(const FrameParams* __restrict__ fpp, DeviceScene s, Paths P,
     Counters* counters) {
-    __shared__ RestirShared sh;
+    __shared__ RestirShared<kPbr> sh;
+    __shared__ pbr::Mat mats[kPbr ? 128 : 1];  // shared, not stack: as in k_scatter
     const FrameParams& fp = *fpp;
     const FrameBufs hist = fp.hist;
     const int count = counters->restir;
     if (count == 0) return;
     int cdf_count = 0;
-    const float* cdf = stage_cdf(fp, s, sh, cdf_count);
+    const float* cdf = stage_cdf<kPbr>(fp, s, sh, cdf_count);
     ShadeCtx ctx{fp, s, 0, 0u, cdf, cdf_count};
     constexpr int bounce = 0;
     const bool bsdf_avail = bounce + 1 < fp.max_bounces;
@@ -860,11 +879,11 @@ __global__ void __launch_bounds__(128, 6) k_restir_ris(const FrameParams* __rest
         const int path = P.restir_queue[i];
         const float4 hr = P.hit[path];
         PathRegs st;
-        load_ray(P, path, st);
+        load_ray(P, path, true, st);
         uint32_t rng = P.rng[path];
         Hit h;
         rebuild_hit<kPbr>(s, hr, st, h);
-        pbr::Mat pm;
+        pbr::Mat& pm = mats[kPbr ? threadIdx.x : 0];
         if constexpr (kPbr) {
             if (h.mtype == 5) openpbr_scattering(s, h, pm);
         }
@@ -887,6 +906,7 @@ __global__ void __launch_bounds__(128, 6) k_restir_ris(const FrameParams* __rest
 template <bool kPbr>
 __global__ void __launch_bounds__(128) k_restir_vis(const FrameParams* __restrict__ fpp, DeviceScene s, Paths P,
     Counters* counters) {
+    __shared__ pbr::Mat mats[kPbr ? 128 : 1];
     const FrameParams& fp = *fpp;
     const FrameBufs hist = fp.hist;
     const int count = counters->vis;
@@ -902,7 +922,8 @@ __global__ void __launch_bounds__(128) k_restir_vis(const FrameParams* __restric
         const ReservoirRec* hres = hist.reservoirs + fp.cam[c].pixel_offset;
         const float4 sq = reservoir_slot(fp, P, fp.cur, c, path)->q[2];
         const Candidate sel{__float_as_int(sq.x), sq.y, sq.z};
-        P.res_src_t[slot] = target_at_previous<kPbr>(ctx, c, load_surface(hres + P.res_src[slot].x), sel, bsdf_avail);
+        P.res_src_t[slot] = target_at_previous<kPbr>(ctx, c, load_surface(hres + P.res_src[slot].x), sel, bsdf_avail,
+            mats[kPbr ? threadIdx.x : 0]);
     }
     count_add(&counters->rays[3], ctx.vis_rays);
     if (ctx.overflow) atomicAdd(&counters->overflow, ctx.overflow);
@@ -911,6 +932,7 @@ __global__ void __launch_bounds__(128) k_restir_vis(const FrameParams* __restric
 template <bool kPbr>
 __global__ void __launch_bounds__(128) k_restir(const FrameParams* __restrict__ fpp, DeviceScene s, Paths P,
     Counters* counters) {
+    __shared__ pbr::Mat mats[kPbr ? 128 : 1];
     const FrameParams& fp = *fpp;
     FrameBufs cur = fp.cur;
     const int count = counters->restir;
@@ -922,11 +944,11 @@ __global__ void __launch_bounds__(128) k_restir(const FrameParams* __restrict__ 
         const int path = P.restir_queue[i];
         const float4 hr = P.hit[path];
         PathRegs st;
-        load_ray(P, path, st);
+        load_ray(P, path, true, st);
         uint32_t rng = P.rng[path];
         Hit h;
         rebuild_hit<kPbr>(s, hr, st, h);
-        pbr::Mat pm;
+        pbr::Mat& pm = mats[kPbr ? threadIdx.x : 0];
         if constexpr (kPbr) {
             if (h.mtype == 5) openpbr_scattering(s, h, pm);
         }

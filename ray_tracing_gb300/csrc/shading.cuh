@@ -257,70 +257,68 @@ RTGB_D void set_face(const float3& d, const float3& outward, Hit& h) {
 // triangle, programs.cu:1421-1547). Re-running the test over (eps, far) picks
 // the same root the traversal accepted, so t, uv and normals are identical.
 template <bool kPbr>
-RTGB_D bool reconstruct_surface(const DeviceScene& s, int code, const float3& o, const float3& d, Hit& h) {
+RTGB_D bool reconstruct_surface(const DeviceScene& s, int code, int slot, const float3& o, const float3& d, Hit& h) {
     const int type = static_cast<unsigned>(code) >> 28;
     const int idx = code & 0x0fffffff;
     h.ptype = type;
     h.pidx = idx;
     h.u = 0.0f;
     h.v = 0.0f;
+    if (type > 2) return false;
+    const PrimRecord r = load_prim(s.prims, slot);
     int mi = -1;
     if (type == 0) {
-        const rtgb_sphere sp = s.spheres[idx];
-        const float3 center = ld3(sp.center);
+        const float3 center = xyz(r.q[0]);
+        const float radius = r.q[0].w;
         float t;
-        if (!sphere_t(center, sp.radius, o, d, kRayEpsilon, kRayFar, t)) return false;
+        if (!sphere_t(center, radius, o, d, kRayEpsilon, kRayFar, t)) return false;
         h.t = t;
         h.pos = add(o, mul(d, t));
-        const float3 outward = divs(sub(h.pos, center), sp.radius);
+        const float3 outward = divs(sub(h.pos, center), radius);
         sphere_uv(outward, h.u, h.v);
         set_face(d, outward, h);
-        mi = sp.material_index;
+        mi = __float_as_int(r.q[1].w);
     } else if (type == 1) {
-        const rtgb_quad q = s.quads[idx];
-        const float3 origin = ld3(q.origin), eu = ld3(q.edge_u), ev = ld3(q.edge_v);
-        const float3 n = cross(eu, ev);
-        const float nls = len_sq(n);
-        if (nls <= 1e-12f) return false;
-        const float3 normal = divs(n, sqrtf(nls));
-        const float3 w = divs(n, nls);
+        // the record's unit normal and n / |n|^2 are the reference's float
+        // operations on the edges (k_prim_records); a degenerate quad's are zero
+        const float3 normal = f3(r.q[0].w, r.q[1].w, r.q[2].w);
         float t, u, v;
-        if (!quad_t(origin, normal, w, eu, ev, o, d, kRayEpsilon, kRayFar, t, u, v)) return false;
+        if (!quad_t(xyz(r.q[0]), normal, xyz(r.q[3]), xyz(r.q[1]), xyz(r.q[2]), o, d, kRayEpsilon, kRayFar, t, u, v)) return false;
         h.t = t;
         h.pos = add(o, mul(d, t));
         h.u = u;
         h.v = v;
         set_face(d, normal, h);
-        mi = q.material_index;
-    } else if (type == 2) {
-        const rtgb_triangle tr = s.triangles[idx];
-        const float3 p0 = ld3(tr.p0), p1 = ld3(tr.p1), p2 = ld3(tr.p2);
-        const float3 e1 = sub(p1, p0), e2 = sub(p2, p0);
+        mi = __ldg(&s.quads[idx].material_index);
+    } else {
+        const float3 e1 = xyz(r.q[1]), e2 = xyz(r.q[2]);
+        const int flags = __float_as_int(r.q[1].w);
         float t, u, v;
-        if (!triangle_t(p0, e1, e2, o, d, kRayEpsilon, kRayFar, t, u, v)) return false;
+        if (!triangle_t(xyz(r.q[0]), e1, e2, o, d, kRayEpsilon, kRayFar, t, u, v)) return false;
         const float3 normal = normalize(cross(e1, e2));
         const float w = 1.0f - u - v;
         h.t = t;
         h.pos = add(o, mul(d, t));
-        if (tr.has_texcoords != 0) {
-            h.u = tr.uv0[0] * w + tr.uv1[0] * u + tr.uv2[0] * v;
-            h.v = tr.uv0[1] * w + tr.uv1[1] * u + tr.uv2[1] * v;
-        } else {
-            h.u = u;
-            h.v = v;
-        }
+        h.u = u;
+        h.v = v;
         set_face(d, normal, h);
-        if (tr.has_vertex_normals != 0) {
-            float3 sh = add(mul(ld3(tr.n0), w), add(mul(ld3(tr.n1), u), mul(ld3(tr.n2), v)));
-            if (!near_zero(sh)) {
-                sh = normalize(sh);
-                if (dot(sh, normal) < 0.0f) sh = mul(sh, -1.0f);
-                h.sn = h.front ? sh : mul(sh, -1.0f);
+        if (flags != 0) {
+            const float4* at = reinterpret_cast<const float4*>(s.tri_attr + slot);
+            const float4 a0 = __ldg(at), a1 = __ldg(at + 1), a2 = __ldg(at + 2), a3 = __ldg(at + 3);
+            if ((flags & kTriTexcoords) != 0) {
+                h.u = a0.w * w + a2.w * u + a3.y * v;
+                h.v = a1.w * w + a3.x * u + a3.z * v;
+            }
+            if ((flags & kTriNormals) != 0) {
+                float3 sh = add(mul(xyz(a0), w), add(mul(xyz(a1), u), mul(xyz(a2), v)));
+                if (!near_zero(sh)) {
+                    sh = normalize(sh);
+                    if (dot(sh, normal) < 0.0f) sh = mul(sh, -1.0f);
+                    h.sn = h.front ? sh : mul(sh, -1.0f);
+                }
             }
         }
-        mi = tr.material_index;
-    } else {
-        return false;
+        mi = __float_as_int(r.q[0].w);
     }
     populate_material<kPbr>(s, mi, h);
     return true;
@@ -813,14 +811,16 @@ RTGB_D LightSample sample_direct(const DeviceScene& s, const Hit& rcv, uint32_t&
         cond = area_pdf(area, d2, ac);
     } else {
         if (light.primitive_index < 0 || light.primitive_index >= s.triangle_count) return smp;
-        const rtgb_triangle t = s.triangles[light.primitive_index];
-        const float3 p0 = ld3(t.p0), p1 = ld3(t.p1), p2 = ld3(t.p2);
+        const float4* lt = s.light_tri + 3ll * li;
+        const float4 l0 = __ldg(lt), l1 = __ldg(lt + 1), l2 = __ldg(lt + 2);
+        const float3 p0 = xyz(l0), p1 = xyz(l1), p2 = xyz(l2);
         float w0 = 0.0f, w1 = 0.0f, w2 = 0.0f;
         const float u0 = rnd(rng);
         const float u1 = rnd(rng);
         sample_uniform_triangle(u0, u1, w0, w1, w2);
         smp.position = add(mul(p0, w0), add(mul(p1, w1), mul(p2, w2)));
-        if (t.has_texcoords != 0) {
+        if (l1.w != 0.0f) {  // has texture coordinates
+            const rtgb_triangle& t = s.triangles[light.primitive_index];
             tu = t.uv0[0] * w0 + t.uv1[0] * w1 + t.uv2[0] * w2;
             tv = t.uv0[1] * w0 + t.uv1[1] * w1 + t.uv2[1] * w2;
         } else {
@@ -831,7 +831,7 @@ RTGB_D LightSample sample_direct(const DeviceScene& s, const Hit& rcv, uint32_t&
         const float da = len(an);
         if (da <= 1e-12f) return smp;
         smp.normal = divs(an, da);
-        smp.material_index = t.material_index;
+        smp.material_index = __float_as_int(l0.w);
         const float3 tl = sub(smp.position, sp);
         const float d2 = len_sq(tl);
         if (d2 <= 1e-12f) return empty_sample();
@@ -918,12 +918,14 @@ RTGB_D LightSample emissive_candidate(const DeviceScene& s, const float3& sp, co
             smp.material_index = q.material_index;
         } else {
             if (light.primitive_index < 0 || light.primitive_index >= s.triangle_count) return empty_sample();
-            const rtgb_triangle t = s.triangles[light.primitive_index];
-            const float3 p0 = ld3(t.p0), p1 = ld3(t.p1), p2 = ld3(t.p2);
+            const float4* lt = s.light_tri + 3ll * li;
+            const float4 l0 = __ldg(lt), l1 = __ldg(lt + 1), l2 = __ldg(lt + 2);
+            const float3 p0 = xyz(l0), p1 = xyz(l1), p2 = xyz(l2);
             float w0 = 0.0f, w1 = 0.0f, w2 = 0.0f;
             sample_uniform_triangle(u0, u1, w0, w1, w2);
             smp.position = add(mul(p0, w0), add(mul(p1, w1), mul(p2, w2)));
-            if (t.has_texcoords != 0) {
+            if (l1.w != 0.0f) {  // has texture coordinates
+                const rtgb_triangle& t = s.triangles[light.primitive_index];
                 tu = t.uv0[0] * w0 + t.uv1[0] * w1 + t.uv2[0] * w2;
                 tv = t.uv0[1] * w0 + t.uv1[1] * w1 + t.uv2[1] * w2;
             } else {
@@ -931,7 +933,7 @@ RTGB_D LightSample emissive_candidate(const DeviceScene& s, const float3& sp, co
                 tv = w2;
             }
             an = cross(sub(p1, p0), sub(p2, p0));
-            smp.material_index = t.material_index;
+            smp.material_index = __float_as_int(l0.w);
         }
         const float alen = len(an);
         if (alen <= 1e-12f) return empty_sample();

@@ -32,7 +32,7 @@ struct Paths {
     uint32_t* rng;
     float4* aux_n;      // bounce-0 shading normal.xyz, w = depth
     float4* aux_a;      // bounce-0 albedo.xyz, w = 1 when captured
-    float4* hit;        // x = t, y = surface/medium code bits (-1 miss), z = analytic light index bits
+    float4* hit;        // x = t, y = surface/medium code bits (-1 miss), z = analytic light index bits, w = leaf slot bits
     float4* sh_o[2];    // shadow ray origin.xyz, w = tmax
     float4* sh_d[2];    // shadow ray direction.xyz
     float4* sh_c[2];    // contribution (throughput * direct).xyz, w = 1 when pending
@@ -110,6 +110,8 @@ struct FrameParams {
     int restir_emissive;   // 1: ReSTIR DI resamples the emissive-geometry lights (opt-in; no reference counterpart)
     int record_paths;
     int sort_from_bounce;  // shade in material-bucket order from this bounce on (INT_MAX: never)
+    int openpbr;           // the scene has OpenPBR materials (paths may enter a random-walk medium)
+    int zero_reservoirs;   // cur.reservoirs may hold a ReSTIR frame's records: k_raygen clears them
     FrameBufs cur;      // this frame's buffers
     FrameBufs hist;     // the previous frame's (ping-pong)
 };
@@ -124,6 +126,7 @@ struct LaunchShape {
 
 // Kernel launchers (wavefront.cu). All are asynchronous on `stream`.
 void launch_analytic_hot(DeviceScene scene, float4* out, cudaStream_t stream);
+void launch_light_tri(DeviceScene scene, float4* out, cudaStream_t stream);
 void launch_camera_dirs(const CameraDev& cam, float4* out, cudaStream_t stream);
 void launch_raygen(const FrameParams* fp, Paths paths, Counters* counters, LaunchShape shape, cudaStream_t stream);
 void launch_trace(const FrameParams* fp, DeviceScene scene, Paths paths, Counters* counters, int bounce,
@@ -182,6 +185,9 @@ void launch_tonemap(const float4* beauty, uint8_t* rgba, long long pixels, cudaS
 // Scene preparation kernels (scene_prep.cu).
 void launch_prim_records(const DeviceScene& scene, PrimRecord* records, float4* aabb_lo, float4* aabb_hi, float pad,
     cudaStream_t stream);
-void launch_gather_records(const PrimRecord* in, const int* order, PrimRecord* out, int n, cudaStream_t stream);
+// Leaf records in slot order (`order`: slot -> primitive, null for a single
+// primitive) and, into `attr`, their triangles' normals and texture coordinates.
+void launch_gather_records(const DeviceScene& scene, const PrimRecord* in, const int* order, PrimRecord* out, TriAttr* attr,
+    int n, cudaStream_t stream);
 
 }  // namespace rtgb
