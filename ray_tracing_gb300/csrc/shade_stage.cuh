@@ -641,6 +641,7 @@ __global__ void __launch_bounds__(kSplit ? kPbrBlock : 128, kSplit ? 768 / kPbrB
             P.codes[static_cast<long long>(path) * fp.max_bounces + bounce] =
                 alight >= 0 ? ((5 << 28) | alight) : code;
         }
+        int nee = 0;  // legacy materials: shadow slots stored; OpenPBR holds them here:
         float4 sh_o[2], sh_d[2], sh_c[2];
         sh_c[0] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         sh_c[1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -695,45 +696,85 @@ __global__ void __launch_bounds__(kSplit ? kPbrBlock : 128, kSplit ? 768 / kPbrB
                     // emitters themselves; its sample fills shadow slot 0 in k_restir
                     const bool emissive_restir = restir_bounce && fp.restir_emissive != 0 && h.mtype != 3
                                                  && s.light_count > 0 && find_light(s, h.ptype, h.pidx) < 0;
-                    // accumulate_direct_light (programs.cu:2249-2280) -> shadow slot 0
-                    if (h.mtype != 3 && s.light_count > 0 && !emissive_restir) {
-                        const LightSample l = sample_direct<kPbr>(s, h, rng);
-                        if (l.valid) {
+                    // Next-event estimation. Legacy materials: one body for both light lists
+                    // (slot 0 accumulate_direct_light, programs.cu:2249-2280, slot 1
+                    // accumulate_analytic_direct_light, :2282-2313), a sample that may
+                    // contribute stored as the slot's shadow ray right away instead of held
+                    // in 24 registers: the final room's shading 2.20 -> 1.90 ms, the Cornell
+                    // box's 1.44 -> 1.39. The OpenPBR evaluation makes that form spill (the
+                    // room's shading 35.1 -> 40.9 ms as one body a slot, 35.7 as a loop that
+                    // costs the terrain 0.5 ms), so there each list keeps its own code.
+                    if constexpr (!kPbr) {
+#pragma unroll 1
+                        for (int slot = 0; slot < 2; ++slot) {
+                            LightSample l = empty_sample();
+                            if (slot == 0) {
+                                if (h.mtype != 3 && s.light_count > 0 && !emissive_restir) l = sample_direct<kPbr>(s, h, rng);
+                            } else if (restir_bounce && fp.restir_emissive == 0) {
+                                // accumulate_restir_analytic_direct_light returns before any
+                                // draw for emitters and light-less scenes (programs.cu:2318-2321)
+                                deferred = h.mtype != 3 && s.analytic_count > 0;
+                            } else if (h.mtype != 3 && s.analytic_count > 0) {
+                                const int li = sample_cdf_guided(s.analytic_cdf, s.analytic_guide, s.analytic_count, rnd(rng));
+                                const float u0 = rnd(rng);
+                                const float u1 = rnd(rng);
+                                l = analytic_candidate(s, h.pos, li, u0, u1);
+                            }
+                            if (!l.valid) continue;
                             float bp = 0.0f;
                             const float3 resp = direct_response<kPbr, true>(h, &pm, st.d, st.thr, l.direction, bp);
-                            if (max_comp(resp) > 0.0f) {
-                                const float max_t = l.infinite ? kRayFar : l.distance - kRayEpsilon * 3.0f;
-                                if (max_t > kRayEpsilon) {
-                                    const float mis = bsdf_avail ? power_heuristic(l.pdf, bp) : 1.0f;
-                                    const float3 direct = mul(mul(l.emission, resp), mis / l.pdf);
-                                    sh_o[0] = f4(add(h.pos, mul(l.direction, kRayEpsilon * 2.0f)), max_t);
-                                    sh_d[0] = f4(l.direction, 0.0f);
-                                    sh_c[0] = f4(mul(st.thr, direct), 1.0f);
+                            if (!(max_comp(resp) > 0.0f)) continue;
+                            const float max_t = l.infinite ? kRayFar : l.distance - kRayEpsilon * 3.0f;
+                            if (!(max_t > kRayEpsilon)) continue;
+                            const float mis = l.delta || !bsdf_avail ? 1.0f : power_heuristic(l.pdf, bp);
+                            const float3 direct = mul(mul(l.emission, resp), mis / l.pdf);
+                            P.sh_o[slot][path] = f4(add(h.pos, mul(l.direction, kRayEpsilon * 2.0f)), max_t);
+                            P.sh_d[slot][path] = f4(l.direction, 0.0f);
+                            P.sh_c[slot][path] = f4(mul(st.thr, direct), 1.0f);
+                            nee |= 1 << slot;
+                        }
+                    }
+                    if constexpr (kPbr) {
+                        // accumulate_direct_light (programs.cu:2249-2280) -> shadow slot 0
+                        if (h.mtype != 3 && s.light_count > 0 && !emissive_restir) {
+                            const LightSample l = sample_direct<kPbr>(s, h, rng);
+                            if (l.valid) {
+                                float bp = 0.0f;
+                                const float3 resp = direct_response<kPbr, true>(h, &pm, st.d, st.thr, l.direction, bp);
+                                if (max_comp(resp) > 0.0f) {
+                                    const float max_t = l.infinite ? kRayFar : l.distance - kRayEpsilon * 3.0f;
+                                    if (max_t > kRayEpsilon) {
+                                        const float mis = bsdf_avail ? power_heuristic(l.pdf, bp) : 1.0f;
+                                        const float3 direct = mul(mul(l.emission, resp), mis / l.pdf);
+                                        sh_o[0] = f4(add(h.pos, mul(l.direction, kRayEpsilon * 2.0f)), max_t);
+                                        sh_d[0] = f4(l.direction, 0.0f);
+                                        sh_c[0] = f4(mul(st.thr, direct), 1.0f);
+                                    }
                                 }
                             }
                         }
-                    }
-                    if (restir_bounce && fp.restir_emissive == 0) {
-                        // accumulate_restir_analytic_direct_light returns before any
-                        // draw for emitters and light-less scenes (programs.cu:2318-2321)
-                        deferred = h.mtype != 3 && s.analytic_count > 0;
-                    } else if (h.mtype != 3 && s.analytic_count > 0) {
-                        // accumulate_analytic_direct_light (programs.cu:2282-2313) -> shadow slot 1
-                        const int li = sample_cdf_guided(s.analytic_cdf, s.analytic_guide, s.analytic_count, rnd(rng));
-                        const float u0 = rnd(rng);
-                        const float u1 = rnd(rng);
-                        const LightSample l = analytic_candidate(s, h.pos, li, u0, u1);
-                        if (l.valid) {
-                            float bp = 0.0f;
-                            const float3 resp = direct_response<kPbr, true>(h, &pm, st.d, st.thr, l.direction, bp);
-                            if (max_comp(resp) > 0.0f) {
-                                const float max_t = l.infinite ? kRayFar : l.distance - kRayEpsilon * 3.0f;
-                                if (max_t > kRayEpsilon) {
-                                    const float mis = l.delta || !bsdf_avail ? 1.0f : power_heuristic(l.pdf, bp);
-                                    const float3 direct = mul(mul(l.emission, resp), mis / l.pdf);
-                                    sh_o[1] = f4(add(h.pos, mul(l.direction, kRayEpsilon * 2.0f)), max_t);
-                                    sh_d[1] = f4(l.direction, 0.0f);
-                                    sh_c[1] = f4(mul(st.thr, direct), 1.0f);
+                        if (restir_bounce && fp.restir_emissive == 0) {
+                            // accumulate_restir_analytic_direct_light returns before any
+                            // draw for emitters and light-less scenes (programs.cu:2318-2321)
+                            deferred = h.mtype != 3 && s.analytic_count > 0;
+                        } else if (h.mtype != 3 && s.analytic_count > 0) {
+                            // accumulate_analytic_direct_light (programs.cu:2282-2313) -> shadow slot 1
+                            const int li = sample_cdf_guided(s.analytic_cdf, s.analytic_guide, s.analytic_count, rnd(rng));
+                            const float u0 = rnd(rng);
+                            const float u1 = rnd(rng);
+                            const LightSample l = analytic_candidate(s, h.pos, li, u0, u1);
+                            if (l.valid) {
+                                float bp = 0.0f;
+                                const float3 resp = direct_response<kPbr, true>(h, &pm, st.d, st.thr, l.direction, bp);
+                                if (max_comp(resp) > 0.0f) {
+                                    const float max_t = l.infinite ? kRayFar : l.distance - kRayEpsilon * 3.0f;
+                                    if (max_t > kRayEpsilon) {
+                                        const float mis = l.delta || !bsdf_avail ? 1.0f : power_heuristic(l.pdf, bp);
+                                        const float3 direct = mul(mul(l.emission, resp), mis / l.pdf);
+                                        sh_o[1] = f4(add(h.pos, mul(l.direction, kRayEpsilon * 2.0f)), max_t);
+                                        sh_d[1] = f4(l.direction, 0.0f);
+                                        sh_c[1] = f4(mul(st.thr, direct), 1.0f);
+                                    }
                                 }
                             }
                         }
@@ -764,14 +805,18 @@ __global__ void __launch_bounds__(kSplit ? kPbrBlock : 128, kSplit ? 768 / kPbrB
         if (deferred) {
             // the NEE slot travels to k_restir, which adds the ReSTIR slot (1 for
             // analytic lights, 0 for emissive geometry) and queues the shadow rays
-            const bool em = fp.restir_emissive != 0;
-            const float4 kc = em ? sh_c[1] : sh_c[0];
-            (em ? P.sh_c[1] : P.sh_c[0])[path] = kc;
-            if (kc.w != 0.0f) {
-                (em ? P.sh_o[1] : P.sh_o[0])[path] = em ? sh_o[1] : sh_o[0];
-                (em ? P.sh_d[1] : P.sh_d[0])[path] = em ? sh_d[1] : sh_d[0];
+            const int kept = fp.restir_emissive != 0 ? 1 : 0;
+            if constexpr (kPbr) {
+                const float4 kc = kept ? sh_c[1] : sh_c[0];
+                P.sh_c[kept][path] = kc;
+                if (kc.w != 0.0f) {
+                    P.sh_o[kept][path] = kept ? sh_o[1] : sh_o[0];
+                    P.sh_d[kept][path] = kept ? sh_d[1] : sh_d[0];
+                }
+            } else if ((nee >> kept & 1) == 0) {
+                P.sh_c[kept][path] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             }
-        } else {
+        } else if constexpr (kPbr) {
             any_shadow = sh_c[0].w != 0.0f || sh_c[1].w != 0.0f;
             for (int k = 0; k < 2; ++k) {
                 if (sh_c[k].w != 0.0f) {
@@ -780,6 +825,9 @@ __global__ void __launch_bounds__(kSplit ? kPbrBlock : 128, kSplit ? 768 / kPbrB
                 }
                 if (any_shadow) P.sh_c[k][path] = sh_c[k];
             }
+        } else {
+            any_shadow = nee != 0;
+            if (any_shadow && nee != 3) P.sh_c[nee == 1 ? 1 : 0][path] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         }
         if constexpr (kSplit) {
             append_pair(P.scatter_queue, P.shadow_queue, &filled->scatter, path, to_scatter, any_shadow);
@@ -857,12 +905,12 @@ RTGB_D const float* stage_cdf(const FrameParams& fp, const DeviceScene& s, Resti
     return shared ? sh.cdf : src;
 }
 
-// Six resident blocks (80 registers) measured fastest among 1, 6, 8 and 10 for
-// legacy materials; the OpenPBR instance, whose evaluation calls spill, takes
-// four (128 registers): the 24-light OpenPBR gallery's ReSTIR bounce 2.15 ms
-// against 2.26 at six and 2.24 at three.
+// Six resident blocks (80 registers) measured fastest among 1, 6, 8 and 10; for
+// OpenPBR scenes four are as good on average (ReSTIR over emissive triangles:
+// terrain 11.3 against 12.4 ms a frame, room 21.0 against 20.0, gallery 11.2
+// against 10.6), three slower.
 template <bool kPbr>
-__global__ void __launch_bounds__(128, kPbr ? 4 : 6) k_restir_ris(const FrameParams* __restrict__ fpp, DeviceScene s, Paths P,
+__global__ void __launch_bounds__(128, 6) k_restir_ris(const FrameParams* __restrict__ fpp, DeviceScene s, Paths P,
     Counters* counters) {
     __shared__ RestirShared<kPbr> sh;
     __shared__ pbr::Mat mats[kPbr ? 128 : 1];  // shared, not stack: as in k_scatter
