@@ -62,12 +62,25 @@ cudaError_t launch_conv_rows(const void* x, int n, int h, int w, int cin, const 
     const void* mask);
 // Whether launch_conv_rows takes (and is the faster for) a width and channel counts.
 bool conv_rows_fits(int w, int cin, int cout);
+// The sum over a layer's per-CTA weight-gradient partials, and where it goes.
+struct WgradReduce {
+    const float* partial;
+    int ctas, cin, cout, cin_used, cout_used;
+    int bias_row;  // the partials carry the bias gradient
+    float* dw;
+    float* db;
+};
 // Weight (cout_used x cin_used x 3 x 3, FP32) and bias gradients of a k_conv3x3
 // layer (denoiser_train.cu); `partial` holds wgrad_partial_bytes of at least
-// min(sms, tiles) CTAs.
+// min(sms, tiles) CTAs. With `later`, the partials' reduction is described there
+// instead of launched (the partials must then stay until it has run).
 cudaError_t launch_conv3x3_wgrad(const void* x, int n, int h, int w, int cin, const void* dy, int cout, int cin_used,
     int cout_used, float* dweight, float* dbias, int* err, int sms, cudaStream_t stream, float* partial,
-    size_t partial_bytes);
+    size_t partial_bytes, WgradReduce* later = nullptr);
+// The reductions that `later` put off (device array), in one launch; `blocks`:
+// the largest wgrad_reduce_blocks among them.
+cudaError_t launch_wgrad_reduce_all(const WgradReduce* tasks, int count, int blocks, cudaStream_t stream);
+int wgrad_reduce_blocks(int cin, int cout);
 size_t wgrad_partial_bytes(int ctas, int cin, int cout);
 
 struct UNet;

@@ -275,8 +275,12 @@ __global__ void __launch_bounds__(kWgradThreads, 1) k_conv3x3_wgrad(const __grid
 // layer of a training step.)
 constexpr int kReduceRuns = 32;
 constexpr int kReduceSlices = 8;
-__global__ void __launch_bounds__(kReduceRuns * kReduceSlices) k_wgrad_reduce(const float* __restrict__ partial, int ctas,
-    int cin, int cout, int cin_used, int cout_used, int bias_row, float* __restrict__ dw, float* __restrict__ db) {
+__device__ __forceinline__ void wgrad_reduce(const WgradReduce& t) {
+    const float* __restrict__ partial = t.partial;
+    const int ctas = t.ctas, cin = t.cin, cout = t.cout, cin_used = t.cin_used, cout_used = t.cout_used;
+    const int bias_row = t.bias_row;
+    float* __restrict__ dw = t.dw;
+    float* __restrict__ db = t.db;
     __shared__ float4 sums[kReduceSlices][kReduceRuns];
     const int run = threadIdx.x % kReduceRuns, slice = threadIdx.x / kReduceRuns;
     const int quads = cout >> 2;
@@ -318,6 +322,13 @@ __global__ void __launch_bounds__(kReduceRuns * kReduceSlices) k_wgrad_reduce(co
             dw[(static_cast<long long>(o) * cin_used + i) * 9 + tap] = out[k];
         }
     }
+}
+
+__global__ void __launch_bounds__(kReduceRuns * kReduceSlices) k_wgrad_reduce(WgradReduce task) { wgrad_reduce(task); }
+
+// Every layer of a training step, blockIdx.y the layer (blocks past a layer's end do nothing).
+__global__ void __launch_bounds__(kReduceRuns * kReduceSlices) k_wgrad_reduce_all(const WgradReduce* __restrict__ tasks) {
+    wgrad_reduce(tasks[blockIdx.y]);
 }
 
 // db[o] += sum over pixels of dY (blocked layout, `hw` pixels per image); a
@@ -375,9 +386,22 @@ void set_message(char* msg, size_t cap, const char* text) {
 
 }  // namespace
 
+static int reduce_blocks(int cin, int cout) {
+    const int runs = (9 * cin + 1) * (cout / 4);
+    return (runs + kReduceRuns - 1) / kReduceRuns;
+}
+
+cudaError_t launch_wgrad_reduce_all(const WgradReduce* tasks, int count, int blocks, cudaStream_t stream) {
+    k_wgrad_reduce_all<<<dim3(static_cast<unsigned>(blocks), static_cast<unsigned>(count)), kReduceRuns * kReduceSlices, 0,
+        stream>>>(tasks);
+    return cudaGetLastError();
+}
+
+int wgrad_reduce_blocks(int cin, int cout) { return reduce_blocks(cin, cout); }
+
 cudaError_t launch_conv3x3_wgrad(const void* x, int n, int h, int w, int cin, const void* dy, int cout, int cin_used,
     int cout_used, float* dweight, float* dbias, int* err, int sms, cudaStream_t stream, float* partial,
-    size_t partial_bytes) {
+    size_t partial_bytes, WgradReduce* later) {
     static std::once_flag once;
     static cudaError_t attr = cudaSuccess;
     std::call_once(once, [] {
@@ -401,10 +425,13 @@ cudaError_t launch_conv3x3_wgrad(const void* x, int n, int h, int w, int cin, co
     k_conv3x3_wgrad<<<dim3(gx, gy), kWgradThreads, sh.smem, stream>>>(xmap, ymap, a);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    const int runs = (9 * cin + 1) * (cout / 4);
-    k_wgrad_reduce<<<(runs + kReduceRuns - 1) / kReduceRuns, kReduceRuns * kReduceSlices, 0, stream>>>(partial, gx, cin,
-        cout, cin_used, cout_used, a.ones, dweight, dbias);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    const WgradReduce task{partial, gx, cin, cout, cin_used, cout_used, a.ones, dweight, dbias};
+    if (later != nullptr) {
+        *later = task;
+    } else {
+        k_wgrad_reduce<<<reduce_blocks(cin, cout), kReduceRuns * kReduceSlices, 0, stream>>>(task);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    }
     if (dbias != nullptr && !sh.ones) {
         if ((e = cudaMemsetAsync(dbias, 0, static_cast<size_t>(cout_used) * sizeof(float), stream)) != cudaSuccess) return e;
         const long long hw = static_cast<long long>(h) * w;

@@ -231,6 +231,11 @@ struct Trainer {
     float* zero_bias = nullptr;          // 128 zeros for the input-gradient convolutions
     float* partial = nullptr;
     size_t partial_bytes = 0;
+    size_t partial_at[kLayerCount] = {};
+    WgradReduce reduce_list[kLayerCount] = {};  // what the step's reduction launch sums; the same every step
+    WgradReduce* reduce_tasks = nullptr;        // device copy
+    bool reduce_listed = false;
+    int reduce_blocks = 0;
     // activations (channel-blocked BF16)
     __nv_bfloat16 *t1, *cat1, *p1, *t2, *cat2, *p2, *t3, *t4, *t5, *t6, *out16;
     // gradients
@@ -284,9 +289,13 @@ struct Trainer {
         }
         zero_bias = alloc<float>(128);
         list_pack_tasks();
-        for (const LayerSpec& L : kLayers) {
-            partial_bytes = std::max(partial_bytes, wgrad_partial_bytes(sms, L.cin, L.cout));
+        // a partial buffer per layer: one launch at the end of the backward pass reduces them all
+        for (int l = 0; l < kLayerCount; ++l) {
+            partial_at[l] = partial_bytes / sizeof(float);
+            partial_bytes += (wgrad_partial_bytes(sms, kLayers[l].cin, kLayers[l].cout) + 255) & ~size_t(255);
+            reduce_blocks = std::max(reduce_blocks, wgrad_reduce_blocks(kLayers[l].cin, kLayers[l].cout));
         }
+        reduce_tasks = alloc<WgradReduce>(kLayerCount);
         partial = alloc<float>(partial_bytes / sizeof(float));
         const size_t full = static_cast<size_t>(n) * h * w, half = full / 4, quarter = full / 16;
         t1 = alloc<__nv_bfloat16>(full * 32);
@@ -377,13 +386,23 @@ struct Trainer {
         conv(10, t6, 32, h, w, wf[10], bias[10], 16, 0, out16, 16, 0);
     }
 
-    // weight/bias gradients of layer l (x: its input, dz: its masked output gradient) into the flat vector
+    // weight/bias gradients of layer l (x: its input, dz: its masked output gradient) into its partials;
+    // reduce_gradients sums every layer's into the flat vector
     void wgrad(int l, const void* x, int hh, int ww, const void* dz) {
         const LayerSpec& L = kLayers[l];
         float* dw = grads + offset[l];
         check(launch_conv3x3_wgrad(x, n, hh, ww, L.cin, dz, L.cout, L.cin_used, L.cout_used, dw,
-                  dw + static_cast<long long>(L.cout_used) * L.cin_used * 9, err, sms, stream, partial, partial_bytes),
+                  dw + static_cast<long long>(L.cout_used) * L.cin_used * 9, err, sms, stream, partial + partial_at[l],
+                  wgrad_partial_bytes(sms, L.cin, L.cout), &reduce_list[l]),
             "wgrad");
+    }
+
+    void reduce_gradients() {
+        if (!reduce_listed) {
+            check(cudaMemcpyAsync(reduce_tasks, reduce_list, sizeof reduce_list, cudaMemcpyHostToDevice, stream), "reduce");
+            reduce_listed = true;
+        }
+        check(launch_wgrad_reduce_all(reduce_tasks, kLayerCount, reduce_blocks, stream), "reduce");
     }
 
     // input gradient of layer l: dX (cin channels, written at channel xoff of an xcs tensor) from dz (cout
@@ -444,6 +463,7 @@ struct Trainer {
         dgrad(1, g1, h, w, g_t1, 32, 0, t1);
         // e1a (its input needs no gradient)
         wgrad(0, in16, h, w, g_t1);
+        reduce_gradients();
     }
 
     // forward, loss, backward; then Adam when lr > 0. Returns the mean loss.
