@@ -36,8 +36,8 @@
 //     start and end on even rows.
 // Every wait is bounded and a failed role stops the others.
 //
-// The U-Net's eleven layers at 4 x 640x480: 488 us by tiles, 331 us of stage time
-// with packing and unpacking here (d1a, 80 -> 32 channels: 97 -> 54 us; e1a 42 ->
+// The U-Net at 4 x 640x480 (eleven layers, packing, unpacking): 512 us by tiles,
+// 331 us here (d1a, 80 -> 32 channels: 97 -> 54 us; e1a 42 ->
 // 25; the 48 -> 48 layer with upsampling 52 -> 32 with whole-sector stores). What
 // an issuing warp does per row bounds it (about 115 clocks an instruction, then
 // the wait for the row): the same loop run by one lane, its descriptors moved to
@@ -507,9 +507,8 @@ bool conv_rows_fits(int w, int cin, int cout) {
     return row_stages(cin, cout) >= 2 && 8 * w >= 5 * strips * kCols;
 }
 
-cudaError_t launch_conv_rows(const void* x, int n, int h, int w, int cin, const void* weight, const float* bias, int cout,
-    int relu, void* y, int y_channels, int y_offset, int* err, int sms, cudaStream_t stream, void* pool, int up,
-    const void* mask) {
+// Opts every instance into its shared memory (once; call outside stream capture).
+cudaError_t conv_rows_init() {
     static std::once_flag once;
     static cudaError_t attr = cudaSuccess;
     std::call_once(once, [] {
@@ -518,6 +517,13 @@ cudaError_t launch_conv_rows(const void* x, int n, int h, int w, int cin, const 
             if (attr == cudaSuccess) attr = cudaFuncSetAttribute(rows_kernel(c, true), cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
         }
     });
+    return attr;
+}
+
+cudaError_t launch_conv_rows(const void* x, int n, int h, int w, int cin, const void* weight, const float* bias, int cout,
+    int relu, void* y, int y_channels, int y_offset, int* err, int sms, cudaStream_t stream, void* pool, int up,
+    const void* mask) {
+    const cudaError_t attr = conv_rows_init();
     if (attr != cudaSuccess) return attr;
     RowsArgs a{};
     a.x = static_cast<const __nv_bfloat16*>(x);

@@ -887,7 +887,7 @@ bool unet_tune(UNet* unet, Acts* a) {
 }  // namespace
 
 bool unet_prepare(UNet* unet, int n, int h, int w) {
-    if (conv_init() != cudaSuccess) return false;
+    if (conv_init() != cudaSuccess || conv_rows_init() != cudaSuccess) return false;
     Acts* a = unet_buffers(unet, n, h, w);
     if (a == nullptr) return false;
     if (unet->ready && !a->tuned) {

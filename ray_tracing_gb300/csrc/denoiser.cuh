@@ -60,6 +60,7 @@ cudaError_t launch_conv3x3(const CUtensorMap& map, int n, int h, int w, int cin,
 cudaError_t launch_conv_rows(const void* x, int n, int h, int w, int cin, const void* weight, const float* bias, int cout,
     int relu, void* y, int y_channels, int y_offset, int* err, int sms, cudaStream_t stream, void* pool, int up,
     const void* mask);
+cudaError_t conv_rows_init();
 // Whether launch_conv_rows takes (and is the faster for) a width and channel counts.
 bool conv_rows_fits(int w, int cin, int cout);
 // The sum over a layer's per-CTA weight-gradient partials, and where it goes.

@@ -326,7 +326,7 @@ struct Trainer {
         g_t1 = alloc<__nv_bfloat16>(full * 32);
         loss = alloc<double>(2);  // the sum, then the error word: cleared and read as one
         err = reinterpret_cast<int*>(loss + 1);
-        if (conv_init() != cudaSuccess) throw std::string("conv_init");
+        if (conv_init() != cudaSuccess || conv_rows_init() != cudaSuccess) throw std::string("conv_init");
         cudaDeviceSynchronize();
     }
 

@@ -55,8 +55,9 @@ RTGB_D int tile_pixel(int k, int width, int height) {
 // rays, random states and the first queue. The rest of a fresh path's state
 // (unit throughput, no radiance, no previous scatter) is constant and set by
 // k_shade at bounce 0 (load_first) instead of written here and read there:
-// 44 bytes a path instead of 160, 55 -> 14 us for 4 x 640x480 with the
-// reservoirs' clearing left out where they are clear.
+// 44 bytes a path instead of 160. With the reservoirs' clearing left out where
+// they are clear, 4 x 640x480 take 21 us instead of 55, four 1080p cameras 97
+// instead of 379.
 __global__ void __launch_bounds__(256) k_raygen(const FrameParams* __restrict__ fpp, Paths P, Counters* counters) {
     const FrameParams& fp = *fpp;
     const FrameBufs cur = fp.cur;
