@@ -686,7 +686,9 @@ struct rtgb_renderer {
         sample_stream = 0;
         reset_accumulation();
         std::memset(h_counters, 0, sizeof(Counters));
-        RTGB_CHECK(cudaMemsetAsync(d_counters, 0, sizeof(Counters), stream));
+        // The queue lengths behind the host's part are set by every k_raygen;
+        // clearing those 8 KB as well took 3 of the 11 us of an unchanged scene.
+        RTGB_CHECK(cudaMemsetAsync(d_counters, 0, offsetof(Counters, lengths), stream));
         RTGB_CHECK(cudaStreamSynchronize(stream));
     }
 
