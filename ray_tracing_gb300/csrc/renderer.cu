@@ -303,7 +303,8 @@ struct rtgb_renderer {
     uint64_t frame_h2d = 0;
     // graph
     cudaGraphExec_t graph_exec = nullptr;
-    long long graph_key[5] = {-1, -1, -1, -1, -1};
+    static constexpr int kGraphKey = 5 + RTGB_MAX_CAMERAS;
+    long long graph_key[kGraphKey] = {-1};
     // the scene the captured launches carry by value: a refit or an update that
     // leaves every address and count in place keeps the graph
     DeviceScene graph_scene{};
@@ -1307,10 +1308,14 @@ struct rtgb_renderer {
         RTGB_CHECK(cudaMemcpyAsync(d_fp, &fp, sizeof fp, cudaMemcpyHostToDevice, stream));
 
         RTGB_CHECK(cudaEventRecord(ev_start, stream));
-        // the captured launches depend on the bucketing switch too (the sort kernels are in or out)
-        const long long key[5] = {total_paths, mb,
+        // the captured launches depend on the bucketing switch too (the sort kernels are in or out), and
+        // the denoiser's carry its batches' sizes and pixel offsets: every camera's width and height
+        long long key[kGraphKey] = {total_paths, mb,
             static_cast<long long>(paths.ray_o != nullptr) | (fp.sort_from_bounce != INT_MAX ? 2ll : 0ll),
             reinterpret_cast<long long>(scene.prims), (denoise_this_frame ? 1ll : 0ll) | (static_cast<long long>(unet_generation) << 1)};
+        for (int c = 0; c < active && denoise_this_frame; ++c) {
+            key[5 + c] = static_cast<long long>(rig.cameras[c].width) << 32 | rig.cameras[c].height;
+        }
         if (use_graph) {
             if (!graph_exec || std::memcmp(key, graph_key, sizeof key) != 0 ||
                 std::memcmp(&scene, &graph_scene, sizeof scene) != 0) {
