@@ -13,10 +13,9 @@
 #include <limits>
 #include <new>
 #include <string>
-#include <system_error>
-#include <thread>
 #include <vector>
 
+#include "change_hash.h"
 #include "denoiser.cuh"
 #include "lbvh.cuh"
 #include "light_table.cuh"
@@ -460,80 +459,11 @@ struct rtgb_renderer {
         if (surfaces >= (1ll << 28)) throw Invalid{"scene exceeds 2^28 surface primitives"};
     }
 
-    // FNV-1a over 64-bit words in kHashLanes interleaved lanes, the tail byte by
-    // byte, the lanes folded in order. It detects changes the way the geometry
-    // and scene signatures of gpu_scene_acceleration.cpp:116-135 do: every step
-    // is a bijection of its lane's running hash and of the fold's, so inputs
-    // differing in one word always hash differently. One running hash is a
-    // chain of dependent multiplies, 8 bytes per five or so clocks: 13.5 ms of a
-    // million triangles' 108 MB, more than half of preparing them; the lanes'
-    // multiplies overlap.
-    static constexpr int kHashLanes = 8;
-    static uint64_t fnv_words(uint64_t h, const void* data, size_t bytes) {
-        constexpr uint64_t kPrime = 1099511628211ull;
-        const unsigned char* p = static_cast<const unsigned char*>(data);
-        size_t i = 0;
-        if (bytes >= 8 * kHashLanes) {
-            uint64_t lane[kHashLanes];
-            for (int k = 0; k < kHashLanes; ++k) lane[k] = h + static_cast<uint64_t>(k);
-            for (; i + 8 * kHashLanes <= bytes; i += 8 * kHashLanes) {
-                uint64_t w[kHashLanes];
-                std::memcpy(w, p + i, sizeof w);
-                for (int k = 0; k < kHashLanes; ++k) lane[k] = (lane[k] ^ w[k]) * kPrime;
-            }
-            for (int k = 0; k < kHashLanes; ++k) h = (h ^ lane[k]) * kPrime;
-        }
-        for (; i + 8 <= bytes; i += 8) {
-            uint64_t w;
-            std::memcpy(&w, p + i, 8);
-            h = (h ^ w) * kPrime;
-        }
-        for (; i < bytes; ++i) h = (h ^ p[i]) * kPrime;
-        return h;
-    }
-
-    // Arrays of kHashSplit bytes or more are hashed in kHashParts slices on as
-    // many threads and the slices' hashes folded, so the value does not depend
-    // on whether the threads could be started. Below it starting them (some
-    // 20 us each) costs what they save.
-    static constexpr size_t kHashSplit = 4u << 20;
-    static constexpr int kHashParts = 4;
-    static uint64_t fnv_large(uint64_t h, const void* data, size_t bytes) {
-        if (bytes < kHashSplit) return fnv_words(h, data, bytes);
-        const unsigned char* p = static_cast<const unsigned char*>(data);
-        const size_t part = (bytes / kHashParts) & ~size_t(63);
-        uint64_t hash[kHashParts];
-        auto slice = [&](int k) {
-            const size_t from = part * static_cast<size_t>(k);
-            hash[k] = fnv_words(h + static_cast<uint64_t>(k), p + from, k + 1 < kHashParts ? part : bytes - from);
-        };
-        std::thread workers[kHashParts];
-        for (int k = 1; k < kHashParts; ++k) {
-            try {
-                workers[k] = std::thread(slice, k);
-            } catch (const std::system_error&) {  // no thread to be had: this one does the slice
-                slice(k);
-            }
-        }
-        slice(0);
-        for (int k = 1; k < kHashParts; ++k) {
-            if (workers[k].joinable()) workers[k].join();
-        }
-        return fnv_words(h, hash, sizeof hash);
-    }
-
-    template <typename T>
-    static uint64_t fnv_array(uint64_t h, const T* data, long long count) {
-        const long long n = count > 0 && data ? count : 0;
-        h = fnv_words(h, &n, sizeof n);
-        return n > 0 ? fnv_large(h, data, static_cast<size_t>(n) * sizeof(T)) : h;
-    }
-
     static uint64_t geometry_signature(const rtgb_scene& s) {
-        uint64_t h = 14695981039346656037ull;
-        h = fnv_array(h, s.spheres, s.sphere_count);
-        h = fnv_array(h, s.quads, s.quad_count);
-        return fnv_array(h, s.triangles, s.triangle_count);
+        uint64_t h = kHashSeed;
+        h = hash_array(h, s.spheres, s.sphere_count);
+        h = hash_array(h, s.quads, s.quad_count);
+        return hash_array(h, s.triangles, s.triangle_count);
     }
 
     // The mesh set's contribution to the geometry signature: every prototype
@@ -542,13 +472,13 @@ struct rtgb_renderer {
         for (int i = 0; i < m.prototype_count; ++i) {
             const rtgb_mesh_prototype& p = m.prototypes[i];
             const long long t = p.triangle_count;
-            h = fnv_array(h, p.points, 3ll * p.point_count);
-            h = fnv_array(h, p.corner_points, 3 * t);
-            h = fnv_array(h, p.corner_normals, p.corner_normals ? 9 * t : 0);
-            h = fnv_array(h, p.corner_texcoords, p.corner_texcoords ? 6 * t : 0);
-            h = fnv_array(h, p.triangle_materials, t);
+            h = hash_array(h, p.points, 3ll * p.point_count);
+            h = hash_array(h, p.corner_points, 3 * t);
+            h = hash_array(h, p.corner_normals, p.corner_normals ? 9 * t : 0);
+            h = hash_array(h, p.corner_texcoords, p.corner_texcoords ? 6 * t : 0);
+            h = hash_array(h, p.triangle_materials, t);
         }
-        return fnv_array(h, m.instances, m.instance_count);
+        return hash_array(h, m.instances, m.instance_count);
     }
 
     // Checks a mesh set as add_v2_mesh checks a mesh; returns the number of
@@ -640,13 +570,13 @@ struct rtgb_renderer {
     // Everything prepare uploads besides geometry (the packed light list is a
     // function of geometry and materials, so it needs no hash of its own).
     static uint64_t scene_signature(const rtgb_scene& s, uint64_t geometry) {
-        uint64_t h = fnv_words(geometry, s.background, sizeof s.background);
-        h = fnv_array(h, s.media, s.medium_count);
-        h = fnv_array(h, s.textures, s.texture_count);
-        h = fnv_array(h, s.image_texels, 3ll * s.image_texel_count);
-        h = fnv_array(h, s.materials, s.material_count);
-        h = fnv_array(h, s.openpbr_materials, s.openpbr_material_count);
-        return fnv_array(h, s.analytic_lights, s.analytic_light_count);
+        uint64_t h = hash_words(geometry, s.background, sizeof s.background);
+        h = hash_array(h, s.media, s.medium_count);
+        h = hash_array(h, s.textures, s.texture_count);
+        h = hash_array(h, s.image_texels, 3ll * s.image_texel_count);
+        h = hash_array(h, s.materials, s.material_count);
+        h = hash_array(h, s.openpbr_materials, s.openpbr_material_count);
+        return hash_array(h, s.analytic_lights, s.analytic_light_count);
     }
 
     // GpuSceneAcceleration::update + use_prepared_scene: reuse when nothing
