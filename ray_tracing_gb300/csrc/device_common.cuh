@@ -855,18 +855,26 @@ RTGB_D const char* node4_at(const DeviceScene& s, const float4* staged, int stag
     return reinterpret_cast<const char*>(base + static_cast<long long>(kNode4) * node);
 }
 
-RTGB_D void order_keys(unsigned& a, unsigned& b) {
-    const unsigned lo = min(a, b);
-    b = max(a, b);
-    a = lo;
+// Exchanges neighbours out of order (equal ones stay: a network of these is stable).
+RTGB_D void order_pair(unsigned& ka, int& ca, unsigned& kb, int& cb) {
+    const bool swap = kb < ka;
+    const unsigned k = swap ? kb : ka;
+    const int c = swap ? cb : ca;
+    kb = swap ? ka : kb;
+    cb = swap ? ca : cb;
+    ka = k;
+    ca = c;
 }
 
 // Closest hit over the scene's wide BVH: strict t < closest like the
 // reference, so equal-t primitives keep the first one traversed. A node's four
 // boxes are tested together, then its hit leaves (one loop over the lanes'
 // pending leaves instead of one divergent test per child), then the internal
-// children are visited nearest first: their entry distances, the low two
-// mantissa bits replaced by the child's place, sort as integers. Entries wait
+// children are visited nearest first, those entered at the same distance in the
+// node's order: a stable network over (distance, child) pairs. (Keys with the
+// child's place in the distance's low two bits took as long and confused
+// distances up to three units in the last place apart, so which of two equal-t
+// primitives stayed; ranks from six comparisons took 2-5 % of a frame more.) Entries wait
 // on the stack with their distance and are dropped unvisited once a closer hit
 // is known (a child's box lies inside its parent's, so nothing below a box
 // entered past `closest` can be hit before it). Instruction issue and
@@ -916,30 +924,28 @@ RTGB_D int traverse_closest(const DeviceScene& s, const float3& o, const float3&
                 best_slot = slot;
             }
         }
-        unsigned key[4];
+        unsigned key[4];  // entry distances (positive: they order as integers)
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             const bool visit = ((hit & ~leaves) >> k & 1u) != 0 && tn[k] <= closest;
-            key[k] = visit ? (__float_as_uint(tn[k]) & ~3u) | static_cast<unsigned>(k) : 0xffffffffu;
+            key[k] = visit ? __float_as_uint(tn[k]) : 0xffffffffu;
         }
-        order_keys(key[0], key[1]);
-        order_keys(key[2], key[3]);
-        order_keys(key[0], key[2]);
-        order_keys(key[1], key[3]);
-        order_keys(key[1], key[2]);
+        order_pair(key[0], child[0], key[1], child[1]);
+        order_pair(key[2], child[2], key[3], child[3]);
+        order_pair(key[1], child[1], key[2], child[2]);
+        order_pair(key[0], child[0], key[1], child[1]);
+        order_pair(key[2], child[2], key[3], child[3]);
+        order_pair(key[1], child[1], key[2], child[2]);
         if (key[0] != 0xffffffffu) {
             // farthest first onto the stack, continue with the nearest
 #pragma unroll
             for (int k = 3; k >= 1; --k) {
                 if (key[k] != 0xffffffffu) {
-                    if (sp < kTraversalStack) {
-                        stack[sp++] = make_int2(static_cast<int>(key[k] & ~3u), pick4(child, static_cast<int>(key[k] & 3u)));
-                    } else {
-                        ++overflow;
-                    }
+                    if (sp < kTraversalStack) stack[sp++] = make_int2(static_cast<int>(key[k]), child[k]);
+                    else ++overflow;
                 }
             }
-            node = pick4(child, static_cast<int>(key[0] & 3u));
+            node = child[0];
             continue;
         }
         node = -1;
