@@ -48,6 +48,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <cstdint>
 #include <mutex>
 
 #include "denoiser.cuh"
@@ -523,6 +524,8 @@ cudaError_t conv_rows_init() {
 cudaError_t launch_conv_rows(const void* x, int n, int h, int w, int cin, const void* weight, const float* bias, int cout,
     int relu, void* y, int y_channels, int y_offset, int* err, int sms, cudaStream_t stream, void* pool, int up,
     const void* mask) {
+    // a row's bulk copies start on 16-byte boundaries (k_conv3x3's tensor map refuses such an input itself)
+    if ((reinterpret_cast<uintptr_t>(x) & 15u) != 0) return cudaErrorInvalidValue;
     const cudaError_t attr = conv_rows_init();
     if (attr != cudaSuccess) return attr;
     RowsArgs a{};
