@@ -38,11 +38,13 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <cstdint>
 #include <cstdio>
 #include <cstring>
 #include <mutex>
 
 #include "denoiser.cuh"
+#include "per_device.h"
 #include "rtgb.h"
 #include "tc_primitives.cuh"
 
@@ -369,15 +371,31 @@ __global__ void __launch_bounds__(kBiasThreads) k_bias_grad(const __nv_bfloat16*
     (void)n;
 }
 
-struct Scratch {
-    void* p = nullptr;
-    size_t bytes = 0;
-    std::mutex m;
-};
+// Where the single-layer entry point takes its partials from, in stream order and
+// one allocation per call: calls on several streams and devices share nothing.
+// The pool keeps up to the largest layer's partials between calls (45 MB on 152
+// SMs), as a buffer kept for the process would: a call alone takes 4 us more than
+// with such a buffer (64 x 64, 16 -> 16 channels 25 against 21 us), one among
+// others 1 us (16 x 256 x 256, 32 -> 32 channels 73.4 against 71.9).
+constexpr uint64_t kKeptPartials = 64u << 20;
 
-Scratch& wgrad_scratch() {
-    static Scratch s;
-    return s;
+cudaError_t partials_pool(cudaMemPool_t* out) {
+    static OncePerDevice once;
+    static cudaMemPool_t pools[kMaxDevices] = {};
+    int device = 0;
+    cudaError_t e = once.run([](int dev) {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        cudaError_t made = cudaMemPoolCreate(&pools[dev], &props);
+        uint64_t keep = kKeptPartials;
+        if (made == cudaSuccess) made = cudaMemPoolSetAttribute(pools[dev], cudaMemPoolAttrReleaseThreshold, &keep);
+        return made;
+    });
+    if (e == cudaSuccess) e = cudaGetDevice(&device);
+    if (e == cudaSuccess) *out = pools[device];
+    return e;
 }
 
 void set_message(char* msg, size_t cap, const char* text) {
@@ -472,25 +490,21 @@ extern "C" rtgb_status rtgb_conv3x3_wgrad_bf16(const void* x, int32_t n, int32_t
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     sms = sms > 0 ? sms : 1;
-    Scratch& sc = wgrad_scratch();
-    std::lock_guard<std::mutex> lock(sc.m);
-    const size_t need = wgrad_partial_bytes(sms, c_in, c_out);
-    if (sc.bytes < need) {
-        // the previous user of the scratch may still be running on its stream
-        if (sc.p != nullptr) {
-            cudaDeviceSynchronize();
-            cudaFree(sc.p);
-        }
-        sc.p = nullptr;
-        sc.bytes = 0;
-        if (cudaMalloc(&sc.p, need) != cudaSuccess) {
-            set_message(message, message_size, "out of device memory for the weight-gradient partials");
-            return RTGB_RUNTIME_ERROR;
-        }
-        sc.bytes = need;
+    const cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const size_t bytes = wgrad_partial_bytes(sms, c_in, c_out);
+    cudaMemPool_t pool = nullptr;
+    void* partial = nullptr;
+    cudaError_t e = partials_pool(&pool);
+    if (e == cudaSuccess) e = cudaMallocFromPoolAsync(&partial, bytes, pool, st);
+    if (e != cudaSuccess) {
+        (void)cudaGetLastError();
+        set_message(message, message_size, "out of device memory for the weight-gradient partials");
+        return RTGB_RUNTIME_ERROR;
     }
-    const cudaError_t e = launch_conv3x3_wgrad(x, n, h, w, c_in, dy, c_out, c_in, c_out, dweight, dbias, device_error, sms,
-        static_cast<cudaStream_t>(stream), static_cast<float*>(sc.p), sc.bytes);
+    e = launch_conv3x3_wgrad(x, n, h, w, c_in, dy, c_out, c_in, c_out, dweight, dbias, device_error, sms, st,
+        static_cast<float*>(partial), bytes);
+    const cudaError_t freed = cudaFreeAsync(partial, st);
+    if (e == cudaSuccess) e = freed;
     if (e != cudaSuccess) {
         set_message(message, message_size, cudaGetErrorString(e));
         return RTGB_RUNTIME_ERROR;
