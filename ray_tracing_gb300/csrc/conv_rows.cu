@@ -49,9 +49,9 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
-#include <mutex>
 
 #include "denoiser.cuh"
+#include "per_device.h"
 #include "tc_primitives.cuh"
 
 namespace rtgb {
@@ -508,17 +508,17 @@ bool conv_rows_fits(int w, int cin, int cout) {
     return row_stages(cin, cout) >= 2 && 8 * w >= 5 * strips * kCols;
 }
 
-// Opts every instance into its shared memory (once; call outside stream capture).
+// Opts every instance into its shared memory (once per device; call outside
+// stream capture).
 cudaError_t conv_rows_init() {
-    static std::once_flag once;
-    static cudaError_t attr = cudaSuccess;
-    std::call_once(once, [] {
-        for (int c = 16; c <= 64 && attr == cudaSuccess; c += 16) {
-            attr = cudaFuncSetAttribute(rows_kernel(c, false), cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
-            if (attr == cudaSuccess) attr = cudaFuncSetAttribute(rows_kernel(c, true), cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
+    static OncePerDevice once;
+    return once.run([](int) {
+        cudaError_t e = cudaSuccess;
+        for (int k = 0; k < 8 && e == cudaSuccess; ++k) {
+            e = cudaFuncSetAttribute(rows_kernel(16 * (k / 2 + 1), k % 2 != 0), cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
         }
+        return e;
     });
-    return attr;
 }
 
 cudaError_t launch_conv_rows(const void* x, int n, int h, int w, int cin, const void* weight, const float* bias, int cout,

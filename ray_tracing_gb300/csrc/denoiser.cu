@@ -42,11 +42,13 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdio>
 #include <cstring>
 #include <mutex>
 
 #include "denoiser.cuh"
+#include "per_device.h"
 #include "rtgb.h"
 #include "tc_primitives.cuh"
 
@@ -441,24 +443,23 @@ bool blocked_tensor_map(CUtensorMap* map, const void* x, int n, int h, int w, in
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Opts k_conv3x3 into its shared-memory size (once per process; call it
-// outside stream capture).
-int g_conv_regs = 0;  // registers per thread of k_conv3x3 (set by conv_init)
+std::atomic<int> g_conv_regs{0};  // registers per thread of k_conv3x3 (set by conv_init)
 
+// Opts k_conv3x3 into its shared-memory size (once per device; call it
+// outside stream capture).
 cudaError_t conv_init() {
-    static std::once_flag once;
-    static cudaError_t attr = cudaSuccess;
-    std::call_once(once, [] {
-        attr = cudaFuncSetAttribute(k_conv3x3, cudaFuncAttributeMaxDynamicSharedMemorySize, kConvSmem);
-        if (attr == cudaSuccess) {
-            attr = cudaFuncSetAttribute(k_conv3x3, cudaFuncAttributePreferredSharedMemoryCarveout,
+    static OncePerDevice once;
+    return once.run([](int) {
+        cudaError_t e = cudaFuncSetAttribute(k_conv3x3, cudaFuncAttributeMaxDynamicSharedMemorySize, kConvSmem);
+        if (e == cudaSuccess) {
+            e = cudaFuncSetAttribute(k_conv3x3, cudaFuncAttributePreferredSharedMemoryCarveout,
                 cudaSharedmemCarveoutMaxShared);
         }
         cudaFuncAttributes fa{};
-        if (attr == cudaSuccess) attr = cudaFuncGetAttributes(&fa, k_conv3x3);
-        if (attr == cudaSuccess) g_conv_regs = fa.numRegs;
+        if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_conv3x3);
+        if (e == cudaSuccess) g_conv_regs = fa.numRegs;
+        return e;
     });
-    return attr;
 }
 
 // Launches k_conv3x3; `map` must describe x (conv_input_map).
@@ -477,7 +478,8 @@ cudaError_t launch_conv3x3(const CUtensorMap& map, int n, int h, int w, int cin,
     // 2048 threads and 64 K registers
     int per_sm = (228 * 1024) / (smem + 1024);
     const int tmem_fit = static_cast<int>(512u / a.tmem_cols);
-    const int reg_fit = 65536 / ((g_conv_regs > 0 ? g_conv_regs : 255) * kConvThreads);
+    const int regs = g_conv_regs.load();
+    const int reg_fit = 65536 / ((regs > 0 ? regs : 255) * kConvThreads);
     per_sm = per_sm < tmem_fit ? per_sm : tmem_fit;
     per_sm = per_sm < reg_fit ? per_sm : reg_fit;
     per_sm = per_sm < 2048 / kConvThreads ? per_sm : 2048 / kConvThreads;

@@ -41,7 +41,6 @@
 #include <cstdint>
 #include <cstdio>
 #include <cstring>
-#include <mutex>
 
 #include "denoiser.cuh"
 #include "per_device.h"
@@ -420,10 +419,9 @@ int wgrad_reduce_blocks(int cin, int cout) { return reduce_blocks(cin, cout); }
 cudaError_t launch_conv3x3_wgrad(const void* x, int n, int h, int w, int cin, const void* dy, int cout, int cin_used,
     int cout_used, float* dweight, float* dbias, int* err, int sms, cudaStream_t stream, float* partial,
     size_t partial_bytes, WgradReduce* later) {
-    static std::once_flag once;
-    static cudaError_t attr = cudaSuccess;
-    std::call_once(once, [] {
-        attr = cudaFuncSetAttribute(k_conv3x3_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, kWgradSmemMax);
+    static OncePerDevice once;
+    const cudaError_t attr = once.run([](int) {
+        return cudaFuncSetAttribute(k_conv3x3_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, kWgradSmemMax);
     });
     if (attr != cudaSuccess) return attr;
     CUtensorMap xmap, ymap;
