@@ -42,8 +42,9 @@
 // an issuing warp does per row bounds it (about 115 clocks an instruction, then
 // the wait for the row): the same loop run by one lane, its descriptors moved to
 // uniform registers one by one, took 570 us, two groups instead of four 414 us.
-// A width that fills less than five eighths of its strips (below 80 pixels) is
-// faster by tiles: 3 x 100 x 76 training steps 521 against 512 us.
+// conv_rows_fits says which layers take this form; a frame of 1 x 128 x 128 or
+// 1 x 160 x 120, too small to fill the SMs with rows, took 106 and 116 us of
+// denoising by rows alone, 92 by tiles.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -89,8 +90,9 @@ struct RowsArgs {
     int* err;
     int stages, slots;
     int strips, pairs;     // 128-pixel columns of an image, row pairs of a column
-    int run;               // row pairs per group
+    int run;               // row pairs of a group's run
     long long units;       // n * strips * pairs
+    int cta_step, group_step;  // runs from a CTA's first to the next one's, from a group to the next
 };
 
 struct GroupBars {
@@ -333,8 +335,8 @@ __global__ void __launch_bounds__(rows_threads(kChunks), 1) k_conv_rows(RowsArgs
     GroupBars& bar = bars[group];
     uint8_t* ring = rows + group * a.stages * row_bytes;
     const uint32_t tmem = *tmem_slot + static_cast<uint32_t>(group * kTmemCols);
-    // every group's run of row pairs, in grid order
-    const long long first = (static_cast<long long>(blockIdx.x) * kGroups + group) * a.run;
+    // every group's run of row pairs
+    const long long first = (static_cast<long long>(blockIdx.x) * a.cta_step + group * a.group_step) * a.run;
     const long long end = first + a.run < a.units ? first + a.run : a.units;
     auto fail = [&](int code) {
         *stop = 1;
@@ -503,9 +505,36 @@ RowsKernel rows_kernel(int cout, bool pool) {
 
 }  // namespace
 
-bool conv_rows_fits(int w, int cin, int cout) {
-    const int strips = (w + kCols - 1) / kCols;
-    return row_stages(cin, cout) >= 2 && 8 * w >= 5 * strips * kCols;
+// Row pairs of a group's run when every SM's groups share the image's.
+static int rows_run(int n, int h, int w, int cout, int sms) {
+    const long long units = static_cast<long long>(n) * ((w + kCols - 1) / kCols) * ((h + 1) / 2);
+    const long long groups = static_cast<long long>(sms) * rows_groups(cout / 16);
+    return static_cast<int>((units + groups - 1) / groups);
+}
+
+// By rows a layer takes a start of 6-8 us and 2-6 us for each row pair of a run
+// (the groups' runs proceed side by side), by tiles 5-7 us and 0.004-0.018 us a
+// tile of 8 x 16 pixels, both in proportion to the channels; so rows pay from so
+// many tiles on per SM and per row pair of a run, and that counts a width that
+// fills its strips badly as well as a small image. Measured on 152 SMs, tiles
+// against rows: 80 -> 32 channels 10.5 : 11.7 us at 1 x 256 x 256 (3.4 tiles an SM,
+// runs of one), 14.8 : 13.1 at 16 x 64 x 128 (6.7, one), 22.7 : 15.9 at
+// 1 x 360 x 640 (12.1, two), 97 : 53 at 4 x 480 x 640 (63, eight); 48 -> 48 7.7 : 9.4
+// at 1 x 120 x 160 (1.1, one), 13.7 : 14.8 at 2 x 240 x 320 (7.9, three), 17.6 : 15.2
+// at 1 x 360 x 640 (12.1, three); 112 -> 48 15.9 : 17.2 at 1 x 240 x 320 (3.9, two),
+// 26.0 : 22.8 at 2 x 240 x 320; 32 -> 32 at 16 x 256 pixels' height equal at a width of
+// 76 (16.8, four), 1.30x by rows at 128, 0.94x at 130 (two strips), 1.06x at 160.
+// Layers with `fused` pooling or upsampling gain more (rows store both pixels of an
+// upsampled pair at once) and take rows from three quarters of that on: the network
+// at 2 x 640 x 480 226.9 us with it, 228.9 without, from half of it on 4 us more at
+// 1 x 640 x 480.
+bool conv_rows_fits(int n, int h, int w, int cin, int cout, int sms, bool fused) {
+    if (row_stages(cin, cout) < 2) return false;  // two staged rows a group do not fit beside the weights
+    const long long tiles = static_cast<long long>(n) * ((w + 7) / 8) * ((h + 15) / 16);
+    const long long run = rows_run(n, h, w, cout, sms);
+    // hundredths of a tile per SM
+    const long long least = rows_groups(cout / 16) == 4 ? 130 + 420 * run : (cin <= 48 ? 275 : 210) * run;
+    return 100 * tiles > sms * (fused ? least * 3 / 4 : least);
 }
 
 // Opts every instance into its shared memory (once per device; call outside
@@ -551,10 +580,16 @@ cudaError_t launch_conv_rows(const void* x, int n, int h, int w, int cin, const 
     a.strips = (w + kCols - 1) / kCols;
     a.pairs = (h + 1) / 2;
     a.units = static_cast<long long>(n) * a.strips * a.pairs;
-    const long long groups = static_cast<long long>(sms) * cta_groups;
-    a.run = static_cast<int>((a.units + groups - 1) / groups);
-    const long long used = (a.units + a.run - 1) / a.run;
-    const int grid = static_cast<int>((used + cta_groups - 1) / cta_groups);
+    a.run = rows_run(n, h, w, cout, sms);
+    // Runs that leave every SM a group free go to all SMs in turn, a group of each
+    // (640 x 360 pixels 159 -> 154 us of denoising); else neighbouring runs fill a CTA's
+    // groups, which is 1 % faster than runs in turn (1920 x 1080: 504 against 508 us).
+    const long long runs = (a.units + a.run - 1) / a.run;
+    const bool in_turn = runs <= static_cast<long long>(cta_groups - 1) * sms;
+    const long long ctas = in_turn ? (runs < sms ? runs : sms) : (runs + cta_groups - 1) / cta_groups;
+    const int grid = static_cast<int>(ctas);
+    a.cta_step = in_turn ? 1 : cta_groups;
+    a.group_step = in_turn ? grid : 1;
     int smem = kBarBytes + 9 * cin * cout * 2 + cta_groups * a.stages * (cin / 8) * kPitch;
     smem = smem > kSmemMin ? smem : kSmemMin;
     rows_kernel(cout, pool != nullptr)<<<grid, rows_threads(cout / 16), smem, stream>>>(a);

@@ -1,6 +1,6 @@
-// Denoiser convolutions on the sm_103a tensor cores, by tiles: the form narrow
-// images and c_in = 128 with c_out = 64 take (conv_rows_fits); the others run
-// k_conv_rows (conv_rows.cu).
+// Denoiser convolutions on the sm_103a tensor cores, by tiles: the form of layers
+// with few tiles an SM and of those whose weights leave no room for two staged
+// rows (conv_rows_fits); the others run k_conv_rows (conv_rows.cu).
 //
 // k_conv3x3 is an implicit-GEMM 3x3 convolution (stride 1, zero padding 1) over
 // channel-blocked BF16 tensors, [n][c/8][h][w][8] (8 channels innermost, then
@@ -550,11 +550,13 @@ extern "C" rtgb_status rtgb_conv3x3_bf16(const void* x, int32_t n, int32_t h, in
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const cudaError_t e = conv_rows_fits(w, c_in, c_out)
+    sms = sms > 0 ? sms : 1;
+    const cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const cudaError_t e = conv_rows_fits(n, h, w, c_in, c_out, sms, false)
         ? launch_conv_rows(x, n, h, w, c_in, packed_weight, bias, c_out, relu, y, y_channels, y_channel_offset, device_error,
-              sms > 0 ? sms : 1, static_cast<cudaStream_t>(stream), nullptr, 0, nullptr)
-        : launch_conv3x3(map, n, h, w, c_in, packed_weight, bias, c_out, relu, y, y_channels,
-        y_channel_offset, device_error, sms > 0 ? sms : 1, static_cast<cudaStream_t>(stream));
+              sms, st, nullptr, 0, nullptr)
+        : launch_conv3x3(map, n, h, w, c_in, packed_weight, bias, c_out, relu, y, y_channels, y_channel_offset, device_error,
+              sms, st);
     if (e != cudaSuccess) {
         set_message(message, message_size, cudaGetErrorString(e));
         return RTGB_RUNTIME_ERROR;
@@ -851,7 +853,7 @@ bool unet_tune(UNet* unet, Acts* a) {
     for (int li = 0; li < kLayerCount && ok; ++li) {
         const LayerSpec& l = kLayers[li];
         const LayerCall c = layer_call(a, li, a->h, a->w);
-        if (conv_rows_fits(c.ww, l.cin, l.cout)) continue;  // k_conv_rows has no such choice
+        if (conv_rows_fits(a->n, c.hh, c.ww, l.cin, l.cout, sms, c.pool != nullptr || c.up != 0)) continue;  // k_conv_rows has no such choice
         float best = 1e30f;
         int best_s = 0;
         for (int s = 2; s <= kMaxStages; s += 2) {  // even counts: two issuers per CTA
@@ -908,7 +910,7 @@ cudaError_t unet_run(UNet* unet, const FrameParams* fp, long long pixel_offset, 
     const int h2 = (h + 1) / 2, w2 = (w + 1) / 2, h4 = (h2 + 1) / 2, w4 = (w2 + 1) / 2;
     auto conv = [&](int li, int hh, int ww, void* y, int ych, int yoff, void* pool = nullptr, int up = 0) {
         const LayerSpec& l = kLayers[li];
-        if (conv_rows_fits(ww, l.cin, l.cout)) {
+        if (conv_rows_fits(n, hh, ww, l.cin, l.cout, sms, pool != nullptr || up != 0)) {
             return launch_conv_rows(net->inputs[li], n, hh, ww, l.cin, unet->weights[li].p,
                 static_cast<const float*>(unet->biases[li].p), l.cout, l.relu, y, ych, yoff, err, sms, stream, pool, up, nullptr);
         }

@@ -61,8 +61,9 @@ cudaError_t launch_conv_rows(const void* x, int n, int h, int w, int cin, const 
     int relu, void* y, int y_channels, int y_offset, int* err, int sms, cudaStream_t stream, void* pool, int up,
     const void* mask);
 cudaError_t conv_rows_init();
-// Whether launch_conv_rows takes (and is the faster for) a width and channel counts.
-bool conv_rows_fits(int w, int cin, int cout);
+// Whether launch_conv_rows takes a layer and is the faster for it (`fused`: with
+// pooling or upsampling).
+bool conv_rows_fits(int n, int h, int w, int cin, int cout, int sms, bool fused);
 // The sum over a layer's per-CTA weight-gradient partials, and where it goes.
 struct WgradReduce {
     const float* partial;

@@ -359,7 +359,7 @@ struct Trainer {
     // one convolution: input x (cin channels) at hh x ww
     void conv(int l, const void* x, int cin, int hh, int ww, const void* wts, const float* b, int cout, int relu, void* y,
         int ych, int yoff, void* pool = nullptr, int up = 0, const void* relu_of = nullptr) {
-        if (conv_rows_fits(ww, cin, cout)) {
+        if (conv_rows_fits(n, hh, ww, cin, cout, sms, pool != nullptr || up != 0)) {
             check(launch_conv_rows(x, n, hh, ww, cin, wts, b, cout, relu, y, ych, yoff, err, sms, stream, pool, up, relu_of),
                 "conv");
             return;

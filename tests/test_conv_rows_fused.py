@@ -1,8 +1,9 @@
-"""The row form of the denoiser's convolution with its fused epilogues: pooling
-at 32 and 48 channels, nearest upsampling and the training step's ReLU mask, in
-networks wide enough that every resolution runs by rows (a width must fill five
-eighths of its 128-pixel strips). Bounds as test_denoiser_unet,
-test_denoiser_training and test_denoiser_conv."""
+"""The row form of the denoiser's convolution in the sizes it is chosen for
+(enough 8 x 16-pixel tiles an SM for the row pairs of a run): the edges of its
+128-pixel strips, row pairs and runs, and its fused epilogues - pooling at 32
+and 48 channels, nearest upsampling, the training step's ReLU mask - in networks
+where every resolution runs by rows. Bounds as test_denoiser_conv,
+test_denoiser_unet and test_denoiser_training."""
 import ctypes as C
 
 import numpy as np
@@ -16,21 +17,30 @@ from ray_tracing_gb300 import denoiser, scenes
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n,h,w,cin,cout", [
-    (1, 9, 257, 32, 48),
-    (2, 5, 385, 32, 32),
-    (1, 6, 513, 16, 64),
+@pytest.mark.parametrize("n,h,w,cin,cout,relu,ych,yoff", [
+    (100, 1, 80, 16, 32, 1, 32, 0),    # one row: no neighbours above or below
+    (96, 2, 127, 32, 32, 1, 80, 0),    # a strip's last pixel missing
+    (60, 3, 128, 32, 48, 0, 48, 0),    # exactly a strip, an odd height
+    (40, 5, 129, 48, 48, 1, 112, 0),   # a last strip of one pixel
+    (2, 200, 257, 32, 48, 1, 48, 0),
+    (2, 144, 385, 32, 32, 1, 32, 0),
+    (1, 112, 513, 16, 64, 1, 64, 0),
+    (4, 72, 256, 48, 64, 1, 64, 0),
+    (4, 33, 230, 112, 48, 1, 48, 0),   # two row stages
+    (8, 33, 160, 112, 48, 1, 48, 0),
+    (4, 90, 333, 80, 32, 1, 32, 0),
+    (2, 300, 120, 16, 64, 0, 64, 0),
+    (1, 700, 1000, 64, 64, 1, 112, 48),  # long runs over several columns, four TMEM slots
 ])
-def test_last_strip_of_one_pixel(n, h, w, cin, cout):
-    conv.test_conv3x3_matches_torch(n, h, w, cin, cout, 1, cout, 0)
+def test_rows_match_torch(n, h, w, cin, cout, relu, ych, yoff):
+    conv.test_conv3x3_matches_torch(n, h, w, cin, cout, relu, ych, yoff)
 
 
 @pytest.mark.parametrize("cameras,w,h", [
-    (1, 324, 36),   # quarter resolution 81 wide: pooling and upsampling at both levels by rows
-    (2, 320, 20),   # two images
-    (1, 330, 37),   # odd sizes: pooled edges, upsampling by its own kernel
-    (1, 326, 6),    # upsampling into half resolution by its own kernel, into the full one fused
-    (3, 640, 4),
+    (4, 1000, 200),  # pooling and upsampling at both levels by rows
+    (4, 1004, 206),  # upsampling into half resolution by its own kernel, into the full one fused
+    (4, 1002, 201),  # odd sizes: pooled edges, upsampling by its own kernel
+    (1, 648, 360),   # full and half resolution by rows, the quarter by tiles
 ])
 def test_unet_by_rows(cameras, w, h):
     torch = pytest.importorskip("torch")
@@ -64,7 +74,7 @@ def test_unet_by_rows(cameras, w, h):
             assert np.quantile(rel, 0.999) <= 5e-2, f"camera {cam}: 99.9% {np.quantile(rel, 0.999):.2e}"
 
 
-@pytest.mark.parametrize("n,h,w", [(1, 16, 320), (2, 12, 324), (1, 8, 640), (2, 20, 164)])
+@pytest.mark.parametrize("n,h,w", [(4, 200, 1000), (2, 400, 512), (1, 16, 320)])
 def test_gradients_by_rows(n, h, w):
     torch = pytest.importorskip("torch")
     torch.manual_seed(3)

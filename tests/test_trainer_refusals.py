@@ -11,13 +11,13 @@ from ray_tracing_gb300 import abi, denoiser
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("w", [40, 96, 320])  # tiles; rows at full resolution; rows everywhere
+@pytest.mark.parametrize("h,w", [(8, 40), (8, 320), (128, 1024)])  # by tiles; by tiles; by rows
 @pytest.mark.parametrize("shift", [1, 4])     # elements of two bytes
-def test_misaligned_input_is_refused(w, shift):
+def test_misaligned_input_is_refused(h, w, shift):
     torch = pytest.importorskip("torch")
     torch.manual_seed(3)
     flat = denoiser.flatten(denoiser.build_model()).astype(np.float32)
-    n, h = 1, 8
+    n = 1
     x, t = training._batch(np.random.default_rng(5), n, h, w)
     dev = torch.device("cuda", 0)
     flat_x = torch.from_numpy(training._blocked(x)).to(dev).to(torch.bfloat16).reshape(-1)
