@@ -146,6 +146,13 @@ struct DevBuf {
         bytes = need;
         return p;
     }
+    // As ensure, but gives back what a scene more than four times larger left
+    // behind (smaller buffers stay: allocating again costs more than they hold).
+    void* ensure_fit(size_t need) {
+        if (bytes > kKeptWorkspace && bytes / 4 > need) release();
+        return ensure(need);
+    }
+    static constexpr size_t kKeptWorkspace = 64u << 20;
     template <typename T>
     T* as() const {
         return static_cast<T*>(p);
@@ -240,7 +247,8 @@ struct rtgb_renderer {
     int node4_count = 0;
     // scene preparation's workspaces, kept between prepares (allocating and
     // freeing them, with the synchronisation a free implies, was 0.5 ms of a
-    // refit of 200,000 triangles); the light BVH reuses the scene's
+    // refit of 200,000 triangles) and given back to a much smaller scene
+    // (DevBuf::ensure_fit): 172 bytes a primitive; the light BVH reuses the scene's
     DevBuf lbvh_mem, collapse_mem, unsorted, light_mem;
     bool accel_valid = false;
     int accel_counts[3] = {-1, -1, -1};
@@ -699,7 +707,7 @@ struct rtgb_renderer {
                 static_cast<float*>(light_cdf.ensure((prims + 1) * sizeof(float))), ints(light_guide, kGuide + 1),
                 ints(sphere_light, static_cast<size_t>(d.sphere_count)), ints(quad_light, static_cast<size_t>(d.quad_count)),
                 ints(triangle_light, static_cast<size_t>(d.triangle_count)), ints(light_counts, 4)};
-            RTGB_CHECK(launch_light_table(src, lt, light_mem.ensure(light_table_scratch_bytes(static_cast<long long>(prims))), stream));
+            RTGB_CHECK(launch_light_table(src, lt, light_mem.ensure_fit(light_table_scratch_bytes(static_cast<long long>(prims))), stream));
             int counts[2] = {0, -1};
             RTGB_CHECK(cudaMemcpyAsync(counts, lt.counts, sizeof counts, cudaMemcpyDeviceToHost, stream));
             RTGB_CHECK(cudaStreamSynchronize(stream));
@@ -766,12 +774,12 @@ struct rtgb_renderer {
         const float pad = 1e-5f + 1e-5f * scale;
         d.prim_count = n;
         prim_count = n;
-        unsorted.ensure(static_cast<size_t>(n) * sizeof(PrimRecord));
-        LbvhScratch ls = lbvh_carve(lbvh_mem.ensure(lbvh_scratch_bytes(n)), n);
+        unsorted.ensure_fit(static_cast<size_t>(n) * sizeof(PrimRecord));
+        LbvhScratch ls = lbvh_carve(lbvh_mem.ensure_fit(lbvh_scratch_bytes(n)), n);
         PrimRecord* recs = static_cast<PrimRecord*>(prims.ensure(static_cast<size_t>(n) * sizeof(PrimRecord)));
-        TriAttr* attr = d.triangle_count > 0
-                            ? static_cast<TriAttr*>(tri_attr.ensure(static_cast<size_t>(n) * sizeof(TriAttr)))
-                            : nullptr;
+        TriAttr* attr = nullptr;
+        if (d.triangle_count > 0) attr = static_cast<TriAttr*>(tri_attr.ensure_fit(static_cast<size_t>(n) * sizeof(TriAttr)));
+        else tri_attr.release();
         d.tri_attr = attr;
         launch_prim_records(d, unsorted.as<PrimRecord>(), ls.aabb_lo, ls.aabb_hi, pad, stream);
         RTGB_CHECK(cudaGetLastError());
@@ -802,7 +810,7 @@ struct rtgb_renderer {
             RTGB_CHECK(cudaMemcpyAsync(bvh_parent.p, ls.parent, (2 * static_cast<size_t>(n) - 1) * sizeof(int),
                 cudaMemcpyDeviceToDevice, stream));
             // the wide BVH: the binary hierarchy collapsed, then its boxes filled in
-            void* work = collapse_mem.ensure(collapse_scratch_bytes(n));
+            void* work = collapse_mem.ensure_fit(collapse_scratch_bytes(n));
             const int* count4 = nullptr;
             RTGB_CHECK(number_bvh4(ls.parent, n, work, &count4, stream));
             RTGB_CHECK(cudaMemcpyAsync(&node4_count, count4, sizeof node4_count, cudaMemcpyDeviceToHost, stream));
