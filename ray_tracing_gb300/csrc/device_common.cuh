@@ -855,15 +855,16 @@ RTGB_D const char* node4_at(const DeviceScene& s, const float4* staged, int stag
     return reinterpret_cast<const char*>(base + static_cast<long long>(kNode4) * node);
 }
 
-// Exchanges neighbours out of order (equal ones stay: a network of these is stable).
-RTGB_D void order_pair(unsigned& ka, int& ca, unsigned& kb, int& cb) {
-    const bool swap = kb < ka;
+// Exchanges a pair out of order (with `equal_too`, also an equal one); whether it did.
+RTGB_D bool order_pair(unsigned& ka, int& ca, unsigned& kb, int& cb, bool equal_too) {
+    const bool swap = equal_too ? kb <= ka : kb < ka;
     const unsigned k = swap ? kb : ka;
     const int c = swap ? cb : ca;
     kb = swap ? ka : kb;
     cb = swap ? ca : cb;
     ka = k;
     ca = c;
+    return swap;
 }
 
 // Closest hit over the scene's wide BVH: strict t < closest like the
@@ -871,10 +872,13 @@ RTGB_D void order_pair(unsigned& ka, int& ca, unsigned& kb, int& cb) {
 // boxes are tested together, then its hit leaves (one loop over the lanes'
 // pending leaves instead of one divergent test per child), then the internal
 // children are visited nearest first, those entered at the same distance in the
-// node's order: a stable network over (distance, child) pairs. (Keys with the
-// child's place in the distance's low two bits took as long and confused
+// node's order: five exchanges of (distance, child) pairs, stable by the last
+// one's rule. (Keys with the child's place in the distance's low two bits confused
 // distances up to three units in the last place apart, so which of two equal-t
-// primitives stayed; ranks from six comparisons took 2-5 % of a frame more.) Entries wait
+// primitives stayed; they took 3.15 ms a frame of the Cornell box where this takes
+// 3.16, 6.58 where this takes 6.50 on the terrain and 79.2 where this takes 78.3 in
+// the room. Six exchanges of neighbours took 3.17 ms of the Cornell box, ranks from
+// six comparisons 2-5 % more of every frame.) Entries wait
 // on the stack with their distance and are dropped unvisited once a closer hit
 // is known (a child's box lies inside its parent's, so nothing below a box
 // entered past `closest` can be hit before it). Instruction issue and
@@ -930,12 +934,12 @@ RTGB_D int traverse_closest(const DeviceScene& s, const float3& o, const float3&
             const bool visit = ((hit & ~leaves) >> k & 1u) != 0 && tn[k] <= closest;
             key[k] = visit ? __float_as_uint(tn[k]) : 0xffffffffu;
         }
-        order_pair(key[0], child[0], key[1], child[1]);
-        order_pair(key[2], child[2], key[3], child[3]);
-        order_pair(key[1], child[1], key[2], child[2]);
-        order_pair(key[0], child[0], key[1], child[1]);
-        order_pair(key[2], child[2], key[3], child[3]);
-        order_pair(key[1], child[1], key[2], child[2]);
+        order_pair(key[0], child[0], key[1], child[1], false);
+        order_pair(key[2], child[2], key[3], child[3], false);
+        const bool low = order_pair(key[0], child[0], key[2], child[2], false);
+        const bool high = order_pair(key[1], child[1], key[3], child[3], false);
+        // between them the larger of the two first and the smaller of the two second; equal, the first pair's goes first
+        order_pair(key[1], child[1], key[2], child[2], low || high);
         if (key[0] != 0xffffffffu) {
             // farthest first onto the stack, continue with the nearest
 #pragma unroll
