@@ -336,7 +336,7 @@ __global__ void __launch_bounds__(rows_threads(kChunks), 1) k_conv_rows(RowsArgs
     uint8_t* ring = rows + group * a.stages * row_bytes;
     const uint32_t tmem = *tmem_slot + static_cast<uint32_t>(group * kTmemCols);
     // every group's run of row pairs
-    const long long first = (static_cast<long long>(blockIdx.x) * a.cta_step + group * a.group_step) * a.run;
+    const long long first = static_cast<long long>(static_cast<int>(blockIdx.x) * a.cta_step + group * a.group_step) * a.run;
     const long long end = first + a.run < a.units ? first + a.run : a.units;
     auto fail = [&](int code) {
         *stop = 1;
@@ -522,18 +522,18 @@ static int rows_run(int n, int h, int w, int cout, int sms) {
 // 1 x 360 x 640 (12.1, two), 97 : 53 at 4 x 480 x 640 (63, eight); 48 -> 48 7.7 : 9.4
 // at 1 x 120 x 160 (1.1, one), 13.7 : 14.8 at 2 x 240 x 320 (7.9, three), 17.6 : 15.2
 // at 1 x 360 x 640 (12.1, three); 112 -> 48 15.9 : 17.2 at 1 x 240 x 320 (3.9, two),
-// 26.0 : 22.8 at 2 x 240 x 320; 32 -> 32 at 16 x 256 pixels' height equal at a width of
-// 76 (16.8, four), 1.30x by rows at 128, 0.94x at 130 (two strips), 1.06x at 160.
-// Layers with `fused` pooling or upsampling gain more (rows store both pixels of an
-// upsampled pair at once) and take rows from three quarters of that on: the network
-// at 2 x 640 x 480 226.9 us with it, 228.9 without, from half of it on 4 us more at
-// 1 x 640 x 480.
+// 26.0 : 22.8 at 2 x 240 x 320; 48 -> 64 10.2 : 9.9 at 2 x 120 x 160 (2.1, one); 32 -> 32
+// in 16 images 256 high equal at a width of 76 (16.8, four), 1.30x by rows at 128, 0.94x
+// at 130 (two strips), 1.06x at 160. Layers with `fused` pooling or upsampling gain
+// more (rows store both pixels of an upsampled pair at once) and take rows from three
+// quarters of that on: the network at 2 x 640 x 480 takes 2 us less with it, from half
+// of it on the one at 1 x 640 x 480 4 us more.
 bool conv_rows_fits(int n, int h, int w, int cin, int cout, int sms, bool fused) {
     if (row_stages(cin, cout) < 2) return false;  // two staged rows a group do not fit beside the weights
     const long long tiles = static_cast<long long>(n) * ((w + 7) / 8) * ((h + 15) / 16);
     const long long run = rows_run(n, h, w, cout, sms);
     // hundredths of a tile per SM
-    const long long least = rows_groups(cout / 16) == 4 ? 130 + 420 * run : (cin <= 48 ? 275 : 210) * run;
+    const long long least = rows_groups(cout / 16) == 4 ? 130 + 420 * run : (cin <= 48 && cout <= 48 ? 275 : 210) * run;
     return 100 * tiles > sms * (fused ? least * 3 / 4 : least);
 }
 
