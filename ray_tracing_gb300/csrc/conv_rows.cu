@@ -36,12 +36,15 @@
 //     start and end on even rows.
 // Every wait is bounded and a failed role stops the others.
 //
-// The U-Net at 4 x 640x480 (eleven layers, packing, unpacking): 512 us by tiles,
-// 331 us here (d1a, 80 -> 32 channels: 97 -> 54 us; e1a 42 ->
-// 25; the 48 -> 48 layer with upsampling 52 -> 32 with whole-sector stores). What
-// an issuing warp does per row bounds it (about 115 clocks an instruction, then
-// the wait for the row): the same loop run by one lane, its descriptors moved to
-// uniform registers one by one, took 570 us, two groups instead of four 414 us.
+// The U-Net at 4 x 640x480 (eleven layers, packing, unpacking): 502 us by tiles,
+// 337 us here (d1a, 80 -> 32 channels: 97 -> 54 us; e1a 42 -> 25; the 48 -> 48 layer
+// with upsampling 52 -> 32 with whole-sector stores). d1a issues 242,000
+// instructions (every second row's go in two parts around the slot ring's end), 58
+// clocks apiece an SM: the shared-memory reads of their operands (4 KB of pixels and
+// up to 3 KB of weights at 128 bytes a clock) and the DRAM stream (62 % of its peak)
+// are what is left near a limit, the tensor pipe is at 48 %. The same loop run by
+// one lane, its descriptors moved to uniform registers one by one, took 570 us, two
+// groups instead of four 414 us.
 // conv_rows_fits says which layers take this form; a frame of 1 x 128 x 128 or
 // 1 x 160 x 120, too small to fill the SMs with rows, took 106 and 116 us of
 // denoising by rows alone, 92 by tiles.

@@ -20,8 +20,8 @@ constexpr int kFlagDelta = 2;
 // Threads of a block of the OpenPBR shade kernels, started together for every
 // path (a barrier an iteration): warps that walk the same long code at the same
 // time share its instruction fetches. Against 128 threads without barriers the
-// 1 M-triangle terrain's first shade stage takes 1.31 instead of 1.51 ms and the
-// gallery's frame 4.91 instead of 5.08; 384 threads measure the same, 768 worse.
+// 1 M-triangle terrain's first shade stage takes 1.31 instead of 1.51 ms; 384
+// threads measure the same, 768 worse.
 constexpr int kPbrBlock = 256;
 
 RTGB_D int camera_of_path(const FrameParams& fp, long long path) {
