@@ -20,6 +20,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -353,7 +354,7 @@ struct Trainer {
         }
         pack_tasks = alloc<PackTask>(tasks.size());
         pack_count = static_cast<int>(tasks.size());
-        cudaMemcpy(pack_tasks, tasks.data(), tasks.size() * sizeof(PackTask), cudaMemcpyHostToDevice);
+        check(cudaMemcpy(pack_tasks, tasks.data(), tasks.size() * sizeof(PackTask), cudaMemcpyHostToDevice), "pack tasks");
     }
 
     // one convolution: input x (cin channels) at hh x ww
@@ -506,10 +507,14 @@ rtgb_status rtgb_trainer_create(int32_t n, int32_t h, int32_t w, const float* pa
         return RTGB_INVALID_ARGUMENT;
     }
     *out = nullptr;
-    auto* tr = new rtgb_trainer_s();
+    auto* tr = new (std::nothrow) rtgb_trainer_s();
+    if (tr == nullptr) return RTGB_RUNTIME_ERROR;
     try {
         tr->t.init(n, h, w, params, count);
     } catch (const std::string&) {
+        delete tr;
+        return RTGB_RUNTIME_ERROR;
+    } catch (const std::bad_alloc&) {  // the packing list, an error's text
         delete tr;
         return RTGB_RUNTIME_ERROR;
     }
@@ -526,6 +531,9 @@ rtgb_status rtgb_trainer_step(rtgb_trainer t, const void* input, const float* ta
         if (loss != nullptr) *loss = l;
     } catch (const std::string& e) {
         t->t.error = e;
+        return RTGB_RUNTIME_ERROR;
+    } catch (const std::bad_alloc&) {
+        t->t.error.clear();
         return RTGB_RUNTIME_ERROR;
     }
     return RTGB_OK;
