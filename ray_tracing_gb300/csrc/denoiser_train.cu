@@ -340,7 +340,7 @@ __global__ void __launch_bounds__(kReduceRuns * kReduceSlices) k_wgrad_reduce_al
 constexpr int kBiasThreads = 256;
 constexpr int kBiasLoadsPerThread = 16;
 
-__global__ void __launch_bounds__(kBiasThreads) k_bias_grad(const __nv_bfloat16* __restrict__ dy, int n, long long hw,
+__global__ void __launch_bounds__(kBiasThreads) k_bias_grad(const __nv_bfloat16* __restrict__ dy, long long hw,
     int cout, int cout_used, float* __restrict__ db) {
     __shared__ float part[kBiasThreads / 32][8];
     const int blocks = cout >> 3;
@@ -367,7 +367,6 @@ __global__ void __launch_bounds__(kBiasThreads) k_bias_grad(const __nv_bfloat16*
         for (int w = 0; w < kBiasThreads / 32; ++w) v += part[w][threadIdx.x];
         atomicAdd(db + cb * 8 + threadIdx.x, v);
     }
-    (void)n;
 }
 
 // Where the single-layer entry point takes its partials from, in stream order and
@@ -455,7 +454,7 @@ cudaError_t launch_conv3x3_wgrad(const void* x, int n, int h, int w, int cin, co
         long long bx = (hw + kPerBlock - 1) / kPerBlock;
         bx = bx < 64 ? bx : 64;
         k_bias_grad<<<dim3(static_cast<unsigned>(bx), static_cast<unsigned>(n * (cout >> 3))), kBiasThreads, 0, stream>>>(
-            static_cast<const __nv_bfloat16*>(dy), n, hw, cout, cout_used, dbias);
+            static_cast<const __nv_bfloat16*>(dy), hw, cout, cout_used, dbias);
         e = cudaGetLastError();
     }
     return e;

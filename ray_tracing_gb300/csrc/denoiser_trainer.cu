@@ -358,7 +358,7 @@ struct Trainer {
     }
 
     // one convolution: input x (cin channels) at hh x ww
-    void conv(int l, const void* x, int cin, int hh, int ww, const void* wts, const float* b, int cout, int relu, void* y,
+    void conv(const void* x, int cin, int hh, int ww, const void* wts, const float* b, int cout, int relu, void* y,
         int ych, int yoff, void* pool = nullptr, int up = 0, const void* relu_of = nullptr) {
         if (conv_rows_fits(n, hh, ww, cin, cout, sms, pool != nullptr || up != 0)) {
             check(launch_conv_rows(x, n, hh, ww, cin, wts, b, cout, relu, y, ych, yoff, err, sms, stream, pool, up, relu_of),
@@ -369,22 +369,21 @@ struct Trainer {
         if (!conv_input_map(&map, x, n, hh, ww, cin)) throw std::string("tensor map");
         check(launch_conv3x3(map, n, hh, ww, cin, wts, b, cout, relu, y, ych, yoff, err, sms, stream, pool, up, 0, relu_of),
             "conv");
-        (void)l;
     }
 
     void forward(const void* in16) {
         const int h2 = h / 2, w2 = w / 2, h4 = h / 4, w4 = w / 4;
-        conv(0, in16, 16, h, w, wf[0], bias[0], 32, 1, t1, 32, 0);
-        conv(1, t1, 32, h, w, wf[1], bias[1], 32, 1, cat1, 80, 0, p1);
-        conv(2, p1, 32, h2, w2, wf[2], bias[2], 48, 1, t2, 48, 0);
-        conv(3, t2, 48, h2, w2, wf[3], bias[3], 48, 1, cat2, 112, 0, p2);
-        conv(4, p2, 48, h4, w4, wf[4], bias[4], 64, 1, t3, 64, 0);
-        conv(5, t3, 64, h4, w4, wf[5], bias[5], 64, 1, cat2, 112, 48, nullptr, 1);
-        conv(6, cat2, 112, h2, w2, wf[6], bias[6], 48, 1, t4, 48, 0);
-        conv(7, t4, 48, h2, w2, wf[7], bias[7], 48, 1, cat1, 80, 32, nullptr, 1);
-        conv(8, cat1, 80, h, w, wf[8], bias[8], 32, 1, t5, 32, 0);
-        conv(9, t5, 32, h, w, wf[9], bias[9], 32, 1, t6, 32, 0);
-        conv(10, t6, 32, h, w, wf[10], bias[10], 16, 0, out16, 16, 0);
+        conv(in16, 16, h, w, wf[0], bias[0], 32, 1, t1, 32, 0);
+        conv(t1, 32, h, w, wf[1], bias[1], 32, 1, cat1, 80, 0, p1);
+        conv(p1, 32, h2, w2, wf[2], bias[2], 48, 1, t2, 48, 0);
+        conv(t2, 48, h2, w2, wf[3], bias[3], 48, 1, cat2, 112, 0, p2);
+        conv(p2, 48, h4, w4, wf[4], bias[4], 64, 1, t3, 64, 0);
+        conv(t3, 64, h4, w4, wf[5], bias[5], 64, 1, cat2, 112, 48, nullptr, 1);
+        conv(cat2, 112, h2, w2, wf[6], bias[6], 48, 1, t4, 48, 0);
+        conv(t4, 48, h2, w2, wf[7], bias[7], 48, 1, cat1, 80, 32, nullptr, 1);
+        conv(cat1, 80, h, w, wf[8], bias[8], 32, 1, t5, 32, 0);
+        conv(t5, 32, h, w, wf[9], bias[9], 32, 1, t6, 32, 0);
+        conv(t6, 32, h, w, wf[10], bias[10], 16, 0, out16, 16, 0);
     }
 
     // weight/bias gradients of layer l (x: its input, dz: its masked output gradient) into its partials;
@@ -412,7 +411,7 @@ struct Trainer {
         const LayerSpec& L = kLayers[l];
         for (int k = 0; k * 64 < L.cin; ++k) {
             const int oc = L.cin - 64 * k < 64 ? L.cin - 64 * k : 64;
-            conv(l, dz, L.cout, hh, ww, wb[l][k], zero_bias, oc, 0, dx, xcs, xoff + 64 * k, nullptr, 0, relu_of);
+            conv(dz, L.cout, hh, ww, wb[l][k], zero_bias, oc, 0, dx, xcs, xoff + 64 * k, nullptr, 0, relu_of);
         }
     }
 
